@@ -100,77 +100,141 @@ Win family_window(int kind, int order) {
   return {0, 0, -1, 2}; // ENO
 }
 
-// Prolongation tiles: ptx fine x (<= PTXMAX) by 2*ptyc-1 fine y (ptyc <=
-// pycmax coarse rows) by pz fine z, the widths balanced over the region.
-long long prolong_tiles(Desc &d, int pycmax, int pz) {
-  const int kind = d.kind;
-  long long tot = 1;
-  {
-    const int ntx = (d.n[0] + PTXMAX - 1) / PTXMAX;
-    const int ptx = (d.n[0] + ntx - 1) / ntx;
-    int ptyc = std::min(pycmax, NTHREADS / ptx);
-    const int nty = (d.n[1] + 2 * ptyc - 2) / (2 * ptyc - 1);
-    const int pty = (d.n[1] + nty - 1) / nty;
-    ptyc = std::min(ptyc, (pty + 2) / 2);
-    d.ptx = (unsigned char)ptx;
-    d.ptyc = (unsigned char)ptyc;
-    // the tensor-copy box of a tile's coarse plane: all coarse bases of ptx
-    // fine points, the stencil window, and one point of even-alignment shift
-    const Win w = family_window(kind, d.order);
-    const int W = std::max(w.hi0, w.hi1) - std::min(w.lo0, w.lo1);
-    d.bx = (unsigned char)(((ptx + 2) / 2 + W + 2) & ~1);
-    d.by = (unsigned char)(ptyc + W);
-    d.tiles[0] = (d.n[0] + ptx - 1) / ptx;
-    d.tiles[1] = (d.n[1] + 2 * ptyc - 2) / (2 * ptyc - 1);
-    d.tiles[2] = (d.n[2] + pz - 1) / pz;
-    for (int k = 0; k < 3; ++k) tot *= d.tiles[k];
-  }
-  return tot;
+// phases of the family's lines (Line::push, cgx_device.cuh)
+int family_phases(int kind, int order) {
+  return kind == K_PROLONG_VC || kind == K_PROLONG_CC ? std::max(1, order) : 1;
 }
-
-// Prolongation tiles of the TMA kernels in tile configuration `config`: as
-// prolong_tiles, with as many coarse rows per tile as the configuration's
-// threads (one owner per fine x and coarse row), staged box, x-pass rows and
-// x items allow for the tile's width (the limits of cgx_tma.cuh): in a
-// 128-thread configuration a tile of 16 fine x takes 8 rows, one of 12 takes
-// 10 and one of 6 takes 11 (the x-pass rows' limit).
-long long prolong_tiles_tma(Desc &d, int config) {
-  const TmaCfg &c = TMA_CFGS[config];
+int stencil_width(const Desc &d) {
   const Win w = family_window(d.kind, d.order);
-  const int W = std::max(w.hi0, w.hi1) - std::min(w.lo0, w.lo1);
-  const int ntx = (d.n[0] + PTXMAX - 1) / PTXMAX;
-  const int ptx = (d.n[0] + ntx - 1) / ntx;
-  const int bx = ((ptx + 2) / 2 + W + 2) & ~1;
-  const int xr = TMA_XR, nbx = ptx / 2 + 1, ntl = std::max(1, (int)d.ntl);
-  int rmax = c.nt / ptx;
-  rmax = std::min(rmax, tma_tls(W, c.pyc) / bx - W);
-  rmax = std::min(rmax, (tma_xbuf(W, c.pyc, ntl) / xr - 1) / ntl - W);
-  rmax = std::min(rmax, tma_items(W, c.pyc) / nbx - W);
-  if (rmax < 1) return -1;
-  const int nty = (d.n[1] + 2 * rmax - 2) / (2 * rmax - 1);
-  const int pty = (d.n[1] + nty - 1) / nty;
-  const int ptyc = std::min(rmax, (pty + 2) / 2);
-  d.ptx = (unsigned char)ptx;
-  d.ptyc = (unsigned char)ptyc;
-  d.bx = (unsigned char)bx;
-  d.by = (unsigned char)(ptyc + W);
-  d.tiles[0] = (d.n[0] + ptx - 1) / ptx;
-  d.tiles[1] = (d.n[1] + 2 * ptyc - 2) / (2 * ptyc - 1);
-  d.tiles[2] = (d.n[2] + c.pz - 1) / c.pz;
-  long long tot = 1;
-  for (int k = 0; k < 3; ++k) tot *= d.tiles[k];
-  return tot;
+  return std::max(w.hi0, w.hi1) - std::min(w.lo0, w.lo1);
+}
+int ceil_div(int a, int b) { return (a + b - 1) / b; }
+// Prolongation tiles in tile configuration `config` with at most pzmax fine z
+// points each, the widths balanced over the region.  y and z tiles start at
+// even source positions, so that every coarse row and plane of a tile but the
+// region's first serves two fine points.  A tile takes as many coarse rows as
+// the threads (one owner per fine x and coarse row) and the staged rows (the
+// limits of cgx_tma.cuh) allow for its width: of 128 threads, 8 rows of 16
+// fine x or 10 of 12.  A stage is as many planes as its rows leave room for,
+// balanced over the tile's planes.
+//
+// x tiles start at destination sectors (32 bytes) where the arrays allow it:
+// a store that covers part of a sector makes L2 fetch the rest of it, and
+// 16-wide row pieces that start 16 bytes into a sector write 2.3 instead of
+// 6.3 TB/s.
+//   * every row has the same alignment (pitches of whole sectors): tiles of
+//     16, 12, 8 or 4 points;
+//   * the alignment alternates by half a sector from row to row or plane to
+//     plane (an even row pitch): tiles of 12 points in 16 lanes, two points
+//     further in every other row (d.xs2);
+//   * else, and for a region of one tile in x: at even source positions
+//     where that costs no further tile, which spares a coarse base per row.
+// The sector tiles are taken for one timelevel as long as they do not cost
+// over half again as many tiles (a 32-box order-5 fill of 160^3 boxes: 308 us
+// against 520 us), and for more timelevels, which are bound by their
+// arithmetic, only where they cost none (the boundary slabs of 129^3 levels:
+// 176 us with sector tiles, a tenth more tiles, against 168 us).
+long long prolong_tiles(Desc &d, int config, int pzmax) {
+  const TmaCfg &c = TMA_CFGS[config];
+  const int W = stencil_width(d), ntl = std::min(3, std::max(1, (int)d.ntl));
+  const int fixed = tma_planes(family_phases(d.kind, d.order), ntl); // planes per stage, or 0
+  const int rpt = tma_rpt(W, c.nt, c.pyc, ntl, fixed), tls = tma_tls(W, c.nt, c.pyc, ntl, fixed);
+  const int yo = d.soff[1] & 1, zo = d.soff[2] & 1;
+  const int nu = ceil_div(d.n[0], PTXMAX), po = d.soff[0] & 1;
+  struct XTiles {
+    int ptx, xw, xo, xs2, nbx, bx, nx, ptyc, ny;
+  };
+  auto rows = [&](XTiles x) { // the rest of a choice of x tiles
+    x.bx = tma_bx(x.nbx, W);
+    const int rmax = std::min(c.nt / x.ptx, std::min(rpt, tls / x.bx) / std::max(1, fixed) - W);
+    if (rmax < 1) return x.ny = 0, x;
+    const int nty = ceil_div(d.n[1] + yo, 2 * rmax);
+    x.nx = ceil_div(d.n[0] + x.xo, x.xw);
+    x.ptyc = ceil_div(ceil_div(d.n[1] + yo, nty), 2);
+    x.ny = ceil_div(d.n[1] + yo, 2 * x.ptyc);
+    return x;
+  };
+  auto balanced = [&](int xo, int q) { // ceil((n + xo) / 16) tiles of a multiple of q points
+    const int w = ceil_div(ceil_div(d.n[0] + xo, ceil_div(d.n[0] + xo, PTXMAX)), q) * q;
+    return rows({w, w, xo, 0, q > 1 && (d.soff[0] - xo) % 2 == 0 ? w / 2 : w / 2 + 1});
+  };
+  XTiles x;
+  if (nu == 1) {
+    x = rows({d.n[0], d.n[0], 0, 0, ((d.soff[0] + d.n[0] - 1) >> 1) - (d.soff[0] >> 1) + 1});
+  } else {
+    x = ceil_div(d.n[0] + po, PTXMAX) == nu ? balanced(po, 2) : balanced(0, 1);
+    const long long at = (long long)(reinterpret_cast<uintptr_t>(d.dst) / 8) + d.doff[0] + d.doff[1] * d.dsy + d.doff[2] * d.dsz;
+    const int xo = (int)(at & 3);
+    XTiles s = x;
+    s.ny = 0;
+    if (d.dsy % 4 == 0 && d.dsz % 4 == 0) s = balanced(xo, 4);
+    else if (d.dsy % 2 == 0 && d.dsz % 2 == 0) s = rows({PTXMAX, 12, xo, 2, (d.soff[0] - xo) % 2 == 0 ? 7 : 8});
+    if (s.ny && (x.ny == 0 || (long long)s.nx * s.ny * 2 <= (long long)x.nx * x.ny * (ntl == 1 ? 3 : 2))) x = s;
+  }
+  if (x.ny == 0) return -1;
+  const int by = x.ptyc + W;
+  const int ntz = ceil_div(d.n[2] + zo, pzmax);
+  const int pz = (ceil_div(d.n[2] + zo, ntz) + 1) & ~1;
+  const int planes = pz / 2 + W, pmax = std::min(rpt / by, tls / (x.bx * by));
+  const int stages = ceil_div(planes, fixed ? fixed : pmax);
+  d.ptx = (unsigned char)x.ptx;
+  d.xw = (unsigned char)x.xw;
+  d.xo = (unsigned char)x.xo;
+  d.xs2 = (unsigned char)x.xs2;
+  d.ptyc = (unsigned char)x.ptyc;
+  d.bx = (unsigned char)x.bx;
+  d.by = (unsigned char)by;
+  d.bz = (unsigned char)(fixed ? fixed : ceil_div(planes, stages));
+  d.pz = (short)pz;
+  d.rpx = ceil_div(65536, x.ptx);
+  d.tma = 0;
+  d.tiles[0] = x.nx;
+  d.tiles[1] = x.ny;
+  d.tiles[2] = ceil_div(d.n[2] + zo, pz);
+  division_magic(d.tiles[0], &d.mg[0], &d.sh[0]);
+  division_magic(d.tiles[1], &d.mg[1], &d.sh[1]);
+  return (long long)d.tiles[0] * d.tiles[1] * d.tiles[2];
 }
 
-// Tiles of a descriptor.  Prolongation: the default configuration of
-// prolong_tiles (PTYCMAX rows, PTZ fine z).  Copy and restriction: STILE
-// consecutive points of the flattened region.
+// The most fine z points per tile for prolongation descriptors that run in
+// one launch, by the time that their tiles take on the GPU's CTA slots: a
+// tile costs its coarse planes (pz / 2 and the window's halo) and about four
+// planes' time of set-up and first copies; a launch takes its total over the
+// slots, and one tile at the least.  Many tiles take the configuration's pz
+// (halo planes cost), few are cut in z until the slots are filled: one
+// 64 x 12 x 52 region is 4 tiles of 31 planes uncut and took 78 us.
+constexpr int SM_COUNT = 148;
+int choose_pz(const std::vector<const Desc *> &ds, int config) {
+  int best = TMA_CFGS[config].pz;
+  double best_cost = -1.0;
+  for (int pz = best; pz >= 4; pz /= 2) {
+    double sum = 0.0, longest = 0.0;
+    for (const Desc *p : ds) {
+      Desc d = *p;
+      const long long nt = prolong_tiles(d, config, pz);
+      if (nt <= 0) continue;
+      const double cost = d.pz / 2 + stencil_width(d) + 4;
+      sum += nt * cost;
+      longest = std::max(longest, cost);
+    }
+    const double t = sum / (SM_COUNT * TMA_CFGS[config].mb) + longest;
+    if (best_cost < 0.0 || t < best_cost) {
+      best_cost = t;
+      best = pz;
+    }
+  }
+  return best;
+}
+
+// Tiles of a descriptor launched alone.  Prolongation: the cp.async kernels'
+// configuration.  Copy and restriction: STILE consecutive points of the
+// flattened region.
 int kind_tiles(Desc &d) {
   const int kind = d.kind;
   const bool prol = is_stencil(kind);
   long long tot = 1;
   if (prol) {
-    tot = prolong_tiles(d, PTYCMAX, PTZ);
+    tot = prolong_tiles(d, PLAIN_CFG, choose_pz({&d}, PLAIN_CFG));
   } else {
     const long long npts = (long long)d.n[0] * d.n[1] * d.n[2];
     if (npts >= (1LL << 31)) return -1;
@@ -731,7 +795,7 @@ int launch_pair(const Desc &d, int ntiles, int fp, int *status, cudaStream_t s) 
 using TmaLaunch = int (*)(int, const Desc *, const CUtensorMap *, const int2 *, long long,
                           unsigned long long *, int *, cudaStream_t);
 #define CGX_TMA_ROW(F, P)                                                                      \
-  {klaunch_tma_f##F##_p##P##_c0, klaunch_tma_f##F##_p##P##_c1, klaunch_tma_f##F##_p##P##_c2, \
+  {klaunch_tma_f##F##_p##P##_c0, klaunch_tma_f##F##_p##P##_c1, nullptr, /* tma_kernel_cfg */ \
    klaunch_tma_f##F##_p##P##_c3, klaunch_tma_f##F##_p##P##_c4}
 const TmaLaunch kTmaLaunch[2][2][TMA_NCFG] = {{CGX_TMA_ROW(0, 0), CGX_TMA_ROW(0, 1)},
                                               {CGX_TMA_ROW(1, 0), CGX_TMA_ROW(1, 1)}};
@@ -767,7 +831,7 @@ int launch_map_capped(int fp, const Desc *d, const CUtensorMap *maps, const int2
     if (i < TV_COUNT) {
       const int k = cfg ? cfg[i] : 0;
       if (k < 0 || k >= TMA_NCFG) return fail(CGX_EINVAL, "bad tile configuration %d", k);
-      rc = kTmaLaunch[f][i / 4 >= 5][k](i | (g_debug_skip_tma ? 1 << 30 : 0), d, maps, tm, n, c, status, s);
+      rc = kTmaLaunch[f][i / 4 >= 5][tma_kernel_cfg(k)](i | (g_debug_skip_tma ? 1 << 30 : 0), d, maps, tm, n, c, status, s);
     } else if (i == SEG_STENCIL) {
       rc = f ? klaunch_map_f1(d, tm, n, c, status, s) : klaunch_map_f0(d, tm, n, c, status, s);
     } else {
@@ -795,6 +859,17 @@ PFN_cuTensorMapEncodeTiled_v12000 tma_encoder() {
       cudaGetLastError();
   }
   return fn;
+}
+
+// The tensor-copy unit can address the source arrays of a prolongation that
+// has a TMA variant: 16-byte aligned bases, row and plane pitches that are
+// multiples of 16 bytes.
+bool tma_addressable(const Desc &d) {
+  if (!is_stencil(d.kind) || tma_variant(d) < 0 || !tma_encoder()) return false;
+  if (d.ssy % 2 || d.ssz % 2 || d.ssz >= (1LL << 37)) return false;
+  for (int t = 0; t < d.ntl; ++t)
+    if (reinterpret_cast<uintptr_t>(d.src[t]) % 16) return false;
+  return true;
 }
 
 } // namespace
@@ -1064,21 +1139,25 @@ int cgx_batch_upload(cgx_batch *b, void *stream) {
     else order.push_back((int)i);
   }
   // prolongation descriptors whose arrays TMA can stage are tiled in their
-  // variant's configuration and get tensor maps
+  // variant's configuration and get tensor maps; the others (variant -1) run
+  // in the cp.async form
   std::vector<CUtensorMap> em(3 * b->descs.size());
   std::vector<Desc> dq(b->pdescs);
   std::vector<long long> ntq(b->ntiles.begin(), b->ntiles.end());
-  for (int i : order) {
-    if (!is_stencil(dq[i].kind)) continue;
-    const int v = tma_variant(dq[i]);
-    Desc t = dq[i];
-    long long nt = 0;
-    if (v >= 0) nt = prolong_tiles_tma(t, b->tma_cfg[v]);
-    if (v >= 0 && nt > 0 && nt < (1LL << 31) && encode_tma_maps(t, &em[3 * (size_t)i])) {
-      dq[i] = t;
+  std::map<int, std::vector<int>> by_variant;
+  for (int i : order)
+    if (is_stencil(dq[i].kind)) by_variant[tma_addressable(dq[i]) ? tma_variant(dq[i]) : -1].push_back(i);
+  for (const auto &kv : by_variant) {
+    const int cfg = kv.first >= 0 ? b->tma_cfg[kv.first] : PLAIN_CFG;
+    std::vector<const Desc *> ds;
+    for (int i : kv.second) ds.push_back(&dq[i]);
+    const int pz = choose_pz(ds, cfg);
+    for (int i : kv.second) {
+      const long long nt = prolong_tiles(dq[i], cfg, pz);
+      if (nt <= 0 || nt >= (1LL << 31)) return fail(CGX_EINVAL, "batch: region too large");
       ntq[i] = nt;
-    } else {
-      dq[i].bx = 0;
+      if (kv.first >= 0 && !encode_tma_maps(dq[i], &em[3 * (size_t)i]))
+        return fail(CGX_ECUDA, "batch: a tensor map could not be encoded");
     }
   }
   auto weight = [&](int i) { return (double)b->points[i] / (double)std::max(1LL, ntq[i]); };
@@ -1486,7 +1565,7 @@ int cgx_chain_upload(cgx_chain *c, void *stream) {
           if (order >= 0 && d.order != order)
             return fail(CGX_EUNSUPPORTED, "chain: prolongation orders %d and %d mixed", order, d.order);
           order = d.order;
-          nt = prolong_tiles_tma(d, CFG);
+          nt = prolong_tiles(d, CFG, TMA_CFGS[CFG].pz);
           if (nt <= 0 || nt >= (1LL << 31) || !encode_tma_maps(d, maps))
             return fail(CGX_EUNSUPPORTED,
                         "chain: batch %zu pair %d: the source arrays cannot be staged by TMA "
@@ -1684,6 +1763,9 @@ extern "C" int cgx_transfer_pairs_noalloc(const cgx_pair *pairs, int npairs, voi
                     i0 + i, b.d.order);
       hd[i] = b.d;
       hp[i] = tiles;
+      // a list of many pairs fills the GPU with whole-length tiles
+      if (npairs > SM_COUNT / 8 && is_stencil(b.d.kind))
+        b.ntiles = (int)prolong_tiles(hd[i], PLAIN_CFG, TMA_CFGS[PLAIN_CFG].pz);
       tiles += b.ntiles;
     }
     cudaError_t e = cudaMemcpyAsync(d_descs + i0, hd, n * sizeof(Desc), cudaMemcpyHostToDevice, s);
@@ -1817,26 +1899,23 @@ int launch_tile_map(const Desc *d_descs, const CUtensorMap *d_maps, const int2 *
 // A prolongation descriptor's tiles in TMA tile configuration `config`
 // (the tiling of a batch upload); returns the tile count, <= 0 if none.
 long long tile_prolongation(Desc &d, int config) {
-  return prolong_tiles_tma(d, config);
+  return prolong_tiles(d, config, TMA_CFGS[config].pz);
 }
 
-bool encode_tma_maps(const Desc &d, CUtensorMap maps[3]) {
-  if (!is_stencil(d.kind) || d.bx == 0 || tma_variant(d) < 0) return false;
-  // row and plane pitches must be multiples of 16 bytes
-  if (d.ssy % 2 || d.ssz % 2 || d.ssz >= (1LL << 37)) return false;
+bool encode_tma_maps(Desc &d, CUtensorMap maps[3]) {
+  if (!tma_addressable(d)) return false;
   PFN_cuTensorMapEncodeTiled_v12000 enc = tma_encoder();
-  if (!enc) return false;
   for (int t = 0; t < d.ntl; ++t) {
-    if (reinterpret_cast<uintptr_t>(d.src[t]) % 16) return false;
     const cuuint64_t dims[3] = {(cuuint64_t)d.sext[0], (cuuint64_t)d.sext[1], (cuuint64_t)d.sext[2]};
     const cuuint64_t strides[2] = {(cuuint64_t)d.ssy * 8, (cuuint64_t)d.ssz * 8};
-    const cuuint32_t box[3] = {d.bx, d.by, 1};
+    const cuuint32_t box[3] = {d.bx, d.by, d.bz};
     const cuuint32_t estr[3] = {1, 1, 1};
     CUresult r = enc(&maps[t], CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 3, const_cast<double *>(d.src[t]), dims,
                      strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
                      CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return false;
   }
+  d.tma = 1;
   return true;
 }
 

@@ -96,8 +96,7 @@ __global__ void __launch_bounds__(TMA_CFGS[CFG].nt, TMA_CFGS[CFG].mb)
   __shared__ __align__(16) ChainTile s_ct[4];
   __shared__ __align__(16) Desc s_d[2];
   __shared__ int s_go, s_last;
-  __shared__ __align__(8) uint64_t s_bars[TMA_NB_MAX];
-  __shared__ int s_abort;
+  __shared__ __align__(8) uint64_t s_bars[TMA_NB];
   const int tid = threadIdx.x;
   constexpr int DW = sizeof(Desc) / 16;
   static_assert(sizeof(Desc) % 16 == 0 && DW <= NT, "descriptor staging");
@@ -116,9 +115,8 @@ __global__ void __launch_bounds__(TMA_CFGS[CFG].nt, TMA_CFGS[CFG].mb)
   pdl_wait();
   unsigned long long tn = 0; // thread 0: the claim in flight
   if (tid == 0) {
-    for (int i = 0; i < TMA_NB_MAX; ++i) mbar_init(&s_bars[i], 1);
+    for (int i = 0; i < TMA_NB; ++i) mbar_init(&s_bars[i], 1);
     mbar_fence_init();
-    s_abort = 0;
     for (int k = 0; k < 2; ++k) {
       const long long t = (long long)atomicAdd(&ctl[CHAIN_CLAIM], 1ULL);
       s_idx[k] = t;
@@ -138,7 +136,7 @@ __global__ void __launch_bounds__(TMA_CFGS[CFG].nt, TMA_CFGS[CFG].mb)
     s_go = ok;
   }
   __syncthreads();
-  TmaRing ring{s_bars, &s_abort, 0u};
+  TmaRing ring{s_bars};
   bool ring_ok = true; // false once a TMA wait of this CTA gave up
   for (int i = 0;; ++i) {
     const int slot = i & 3, buf = i & 1;
@@ -162,8 +160,8 @@ __global__ void __launch_bounds__(TMA_CFGS[CFG].nt, TMA_CFGS[CFG].mb)
       if (d.kind == K_PROLONG_VC) {
         const CUtensorMap *m = maps + 3 * (size_t)s_ct[slot].desc;
         const int tile = s_ct[slot].tile;
-        const bool r = d.ntl == 1 ? prolong_tile_tma<VC<ORDER>, FMA, 1, T_NONE, CFG>(d, m, tile, sm, ring, status)
-                                  : prolong_tile_tma<VC<ORDER>, FMA, 3, T_QUAD, CFG>(d, m, tile, sm, ring, status);
+        const bool r = d.ntl == 1 ? prolong_tile<VC<ORDER>, FMA, 1, T_NONE, CFG, true>(d, m, tile, sm, ring, status)
+                                  : prolong_tile<VC<ORDER>, FMA, 3, T_QUAD, CFG, true>(d, m, tile, sm, ring, status);
         if (!r) { // the CTA's ring is no longer in a known state
           ring_ok = false;
           if (tid == 0) atomicExch(&ctl[CHAIN_ABORT], 1ULL);
@@ -216,7 +214,7 @@ __global__ void __launch_bounds__(TMA_CFGS[CFG].nt, TMA_CFGS[CFG].mb)
 }
 
 template <int ORDER, int CFG> constexpr size_t chain_smem_bytes() {
-  return sizeof(double) * TSmem<VC<ORDER>, 3, TMA_CFGS[CFG].pyc, TMA_CFGS[CFG].pd + 2>::total + 128;
+  return sizeof(double) * smem_family<VC<ORDER>, CFG>() + 128;
 }
 
 template <int FMA, int ORDER, int CFG>

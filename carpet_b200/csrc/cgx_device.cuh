@@ -1,10 +1,10 @@
 // cgx_device.cuh -- device side of the grid-transfer kernels (sm_100a, FP64).
 //
 // One descriptor describes one box-pair: a destination region and where its
-// sources lie.  A descriptor is cut into tiles; one CTA of 256 threads runs
-// one tile at a time.  The same tile routines serve the plain per-box kernel
-// (a grid of the pair's tiles) and the persistent batched kernel (tiles taken
-// from a device work queue across many pairs).
+// sources lie.  A descriptor is cut into tiles; one CTA runs one tile at a
+// time.  The same tile routines serve the plain per-box kernel (a grid of the
+// pair's tiles) and the persistent batched kernel (tiles taken from a device
+// work queue across many pairs).
 //
 // Arithmetic follows CarpetLib's operation order exactly (see the operator
 // families below); FMA selects whether each multiply-add is fused
@@ -39,12 +39,10 @@ enum TKind : int { T_NONE = 0, T_LIN = 1, T_QUAD = 2, T_ENO = 3, T_LAG = 4 };
 // Tile geometry.
 constexpr int NTHREADS = 256;
 constexpr int NWARPS = NTHREADS / 32;
-// prolongation: a tile is ptx fine x (at most PTXMAX, so at most 9 coarse
-// bases) by 2*ptyc-1 fine y (at most ptyc coarse rows) by a PTZ chunk of fine
-// z that the CTA marches plane by plane.  ptx and ptyc are chosen per
-// descriptor, balanced over the region; ptx*ptyc <= NTHREADS, one thread per
-// (fine x, coarse y row) column.
-constexpr int PTXMAX = 16, PTYCMAX = 16, PTZ = 64;
+// prolongation: a tile is ptx fine x (at most PTXMAX) by ptyc coarse rows
+// (2*ptyc fine y) by pz fine z, which the CTA marches in stages of bz coarse
+// planes.  The shape is chosen per descriptor (prolong_tiles in cgx.cu).
+constexpr int PTXMAX = 16;
 
 struct Desc {
   int kind, order, ntl, tkind;
@@ -54,10 +52,19 @@ struct Desc {
   int sext[3];  // logical extent of the source arrays (load clamp)
   int tiles[3]; // tile grid over the region
   unsigned char ptx, ptyc; // prolongation tile shape (fine x, coarse y rows)
-  unsigned char bx, by;    // tensor-copy box of a tile's coarse plane; bx = 0: not staged by TMA
+  unsigned char bx, by, bz; // staged coarse box of a stage: points, rows, planes
+  unsigned char tma; // the stages are tensor copies (cgx_tma.cuh)
+  // x tile t: fine points t * xw - xo .. (t + 1) * xw - xo - 1; with xs2, two
+  // points further in the rows of the other sector alignment (prolong_tiles)
+  unsigned char xo, xw;
+  short pz; // fine z points of a tile (even)
+  unsigned char xs2;
+  unsigned char pad0;
+  int rpx; // ceil(65536 / ptx): t / ptx = t * rpx >> 16 for t < 256
+  int pad1;
   long long ssy, ssz; // source strides (elements) in y and z
   long long dsy, dsz; // destination strides
-  unsigned mg[2]; // streaming kinds: division magic for n[0], n[1] (div_magic)
+  unsigned mg[2]; // division magic (div_magic) for n[0], n[1]; prolongation: tiles[0], tiles[1]
   int sh[2];
   const double *src[3];
   double *dst;
@@ -81,6 +88,10 @@ template <int FMA> __device__ __forceinline__ double madd(double a, double b, do
 }
 __device__ __forceinline__ double mul(double a, double b) { return __dmul_rn(a, b); }
 __device__ __forceinline__ double add(double a, double b) { return __dadd_rn(a, b); }
+// madd(a, b, c) for a caller that holds the product ab = mul(a, b)
+template <int FMA> __device__ __forceinline__ double term(double a, double b, double ab, double c) {
+  return FMA ? __fma_rn(a, b, c) : __dadd_rn(ab, c);
+}
 
 // Coefficients as exact dyadic rationals (numerator / 2^k).
 // prolongate_3d_rf2.cc:92-124
@@ -119,6 +130,30 @@ __device__ __forceinline__ double cc_coeff(int order, int di, int m) {
 // axes as interp3(z) of interp2(y) of interp1(x), so the separable passes
 // x -> y -> z reproduce its arithmetic exactly.
 
+// A family evaluates its rule in two forms.  first/next take the window of
+// one fine point at once (get(m): the coarse value at base + m).  Line takes
+// the coarse values of a line one after another: push(v) hands it the value
+// at index j and returns the parity-0 fine value of base j - D0 and the
+// parity-1 value of base j - D1.  The linear families hold no window for it
+// but the partial sums of the N - 1 fine points still open: each new value
+// adds its term to every one of them, which is the reference's own
+// left-to-right order of every sum.  The terms of one push are independent
+// of each other (a window form chains them), a coefficient that stands twice
+// in the stencil costs one product per coarse value instead of two per fine
+// point (in the two-rounding mode, 9 instead of 12 operations of order 5).
+// A sum stays in its register from its first term to its last: push<U> is
+// the push of phase U = (values pushed before) % PHASES.  Values of a sum opened before the
+// line's first point are never read; a caller that knows which of a line's
+// sums it will read gives them as Open, and the others are not formed.
+// FIRST selects the x pass's form of the sum (first).
+
+// The push of value j of a line adds to the sum opened at value j - k its
+// term k; sums opened at values lo .. hi-1 are wanted.
+struct Open {
+  int j = 1 << 20, lo = 0, hi = 1 << 30;
+  __device__ constexpr bool has(int k) const { return j - k >= lo && j - k < hi; }
+};
+
 // vertex-centred Lagrange, prolongate_3d_rf2.cc:151-295
 template <int ORDER> struct VC {
   static constexpr int N = ORDER + 1;
@@ -141,6 +176,28 @@ template <int ORDER> struct VC {
     for (int m = 0; m < N; ++m) r = madd<FMA>(vc_coeff(ORDER, m), get(LO + m), r);
     return r;
   }
+  static constexpr int D0 = 0, D1 = HI, PHASES = N - 1;
+  template <int FMA, bool FIRST> struct Line {
+    double a[N - 1] = {};
+    template <int U>
+    __device__ __forceinline__ void push(double v, double &o0, double &o1, Open w = {}) {
+      double p[N]; // the stencil is symmetric
+#pragma unroll
+      for (int k = 0; k < N; ++k) p[k] = k < N / 2 ? mul(vc_coeff(ORDER, k), v) : p[N - 1 - k];
+      o0 = v;
+      if (w.has(N - 1)) {
+        const double r = term<FMA>(vc_coeff(ORDER, N - 1), v, p[N - 1], a[U]);
+        o1 = FIRST ? add(0.0, r) : r;
+      }
+#pragma unroll
+      for (int k = N - 2; k >= 1; --k)
+        if (w.has(k)) {
+          double &s = a[(U + N - 1 - k) % (N - 1)];
+          s = term<FMA>(vc_coeff(ORDER, k), v, p[k], s);
+        }
+      if (w.has(0)) a[U] = FIRST ? p[0] : term<FMA>(vc_coeff(ORDER, 0), v, p[0], 0.0);
+    }
+  };
 };
 
 // cell-centred Lagrange, prolongate_3d_cc_rf2.cc:150-195: every axis is
@@ -164,6 +221,45 @@ template <int ORDER> struct CC {
   }
   template <int FMA, class G> __device__ __forceinline__ static double first(int par, G get) {
     return next<FMA>(par, get);
+  }
+  static constexpr int D0 = LO0 + N - 1, D1 = HI, PHASES = N > 1 ? N - 1 : 1;
+  template <int FMA, bool FIRST> struct Line {
+    double a[2][PHASES] = {};
+    template <int U>
+    __device__ __forceinline__ void push(double v, double &o0, double &o1, Open w = {}) {
+      double p[2][N], o[2] = {0.0, 0.0}; // the two parities' stencils mirror each other
+#pragma unroll
+      for (int k = 0; k < N; ++k) p[0][k] = p[1][N - 1 - k] = mul(cc_coeff(ORDER, 0, k), v);
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        if (q) w.j -= LO1 - LO0; // parity 1's windows start that much further
+        if (w.has(N - 1)) o[q] = term<FMA>(cc_coeff(ORDER, q, N - 1), v, p[q][N - 1], N > 1 ? a[q][U] : 0.0);
+#pragma unroll
+        for (int k = N - 2; k >= 1; --k)
+          if (w.has(k)) {
+            double &s = a[q][(U + N - 1 - k) % PHASES];
+            s = term<FMA>(cc_coeff(ORDER, q, k), v, p[q][k], s);
+          }
+        if (N > 1 && w.has(0)) a[q][U] = term<FMA>(cc_coeff(ORDER, q, 0), v, p[q][0], 0.0);
+      }
+      o0 = o[0];
+      o1 = o[1];
+    }
+  };
+};
+
+// The limited families are not sums: their Line holds the window's earlier
+// values and evaluates both parities of base j - HI.
+template <class F, int FMA> struct WindowLine {
+  static constexpr int M = F::HI - F::LO;
+  double a[M] = {};
+  template <int U> __device__ __forceinline__ void push(double v, double &o0, double &o1, Open = {}) {
+    auto get = [&](int m) { return m == F::HI ? v : a[m - F::LO]; };
+    o0 = F::template next<FMA>(0, get);
+    o1 = F::template next<FMA>(1, get);
+#pragma unroll
+    for (int k = 0; k + 1 < M; ++k) a[k] = a[k + 1];
+    a[M - 1] = v;
   }
 };
 
@@ -198,6 +294,8 @@ struct ENO {
   template <int FMA, class G> __device__ __forceinline__ static double first(int par, G get) {
     return next<FMA>(par, get);
   }
+  static constexpr int D0 = HI, D1 = HI, PHASES = 1;
+  template <int FMA, bool FIRST> struct Line : WindowLine<ENO, FMA> {};
 };
 
 // cell-centred ENO, prolongate_3d_cc_eno_rf2.cc:198-400 (interp1, interp2
@@ -269,6 +367,8 @@ template <int ORDER> struct CCENO {
   template <int FMA, class G> __device__ __forceinline__ static double first(int par, G get) {
     return next<FMA>(par, get);
   }
+  static constexpr int D0 = HI, D1 = HI, PHASES = 1;
+  template <int FMA, bool FIRST> struct Line : WindowLine<CCENO<ORDER>, FMA> {};
 };
 
 // ---------------------------------------------------------------- time
@@ -707,182 +807,6 @@ __device__ __forceinline__ void restrict_cc5_tile(const D &d, int tile, int lid)
     }
     dst[i + j * d.dsy + k * d.dsz] = r3;
   }
-}
-
-// ---------------------------------------------------------------- prolongation
-// Shared-memory plan per CTA (doubles):
-//   coarse planes  NB x NTL x CY x CXP   (ring buffer filled by cp.async)
-//   x-pass rows    NTL x CY x PTX
-template <class F> struct PGeom {
-  static constexpr int W = F::HI - F::LO;         // window width - 1
-  static constexpr int CX = 16 + W;               // coarse x per plane (16 bases)
-  static constexpr int CXP = CX + (CX % 2 == 0);  // odd row pitch: fewer bank conflicts
-  static constexpr int CY = PTYCMAX + W;          // coarse y per plane
-  static constexpr int Q = W + 1;                 // z window (register queue)
-  static constexpr int PD = 2;                    // prefetch distance (planes)
-  static constexpr int NB = PD + 2;               // staging ring slots
-  static constexpr int XR = 34;                   // x-pass row pitch (2 x 16 + 2)
-};
-template <class F, int NTL> struct PSmem {
-  using G = PGeom<F>;
-  static constexpr int plane = G::CY * G::CXP;
-  static constexpr int coarse = (G::NB * NTL * plane + 1) / 2 * 2; // x-pass rows 16-B aligned
-  static constexpr int xbuf = NTL * G::CY * G::XR; // one plane of x-pass rows
-  static constexpr int total = coarse + 2 * xbuf;   // doubles
-};
-
-template <class F, int FMA, int NTL, int TK, class D>
-__device__ void prolong_tile(D &d, int tile, double *sm) {
-  using G = PGeom<F>;
-  using S = PSmem<F, NTL>;
-  constexpr int LO = F::LO, HI = F::HI, Q = G::Q, W = G::W;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int ptx = d.ptx, ptyc = d.ptyc, pty = 2 * ptyc - 1;
-
-  const int tx = tile % d.tiles[0], rr = tile / d.tiles[0];
-  const int ty = rr % d.tiles[1], tz = rr / d.tiles[1];
-  const int fx0 = tx * ptx, fy0 = ty * pty, fz0 = tz * PTZ;
-  const int nfx = min(ptx, d.n[0] - fx0), nfy = min(pty, d.n[1] - fy0), nfz = min(PTZ, d.n[2] - fz0);
-  // source positions (fine units) of the tile's first points
-  const int sx0 = d.soff[0] + fx0, sy0 = d.soff[1] + fy0, sz0 = d.soff[2] + fz0;
-  // coarse index ranges held in shared memory
-  const int cx0 = (sx0 >> 1) + LO, cx1 = ((sx0 + nfx - 1) >> 1) + HI;
-  const int cy0 = (sy0 >> 1) + LO, cy1 = ((sy0 + nfy - 1) >> 1) + HI;
-  const int cz0 = (sz0 >> 1) + LO, cz1 = ((sz0 + nfz - 1) >> 1) + HI;
-  const int ncx = cx1 - cx0 + 1, ncy = cy1 - cy0 + 1;
-  const int nrows = NTL * ncy; // staged rows per plane: (timelevel, coarse y)
-  const int c_first = sx0 >> 1, c_last = (sx0 + nfx - 1) >> 1;
-  const int xoff = sx0 - 2 * c_first; // fine x of the tile's first point in x-pass rows
-
-  double *coarse = sm;
-  double *xrows = sm + S::coarse;
-
-  // --- staging: warp w copies rows w, w+8, ...; lane = coarse x (< 32)
-  const int gx = cx0 + lane;
-  const bool xin = lane < ncx && gx >= 0 && gx < d.sext[0];
-  auto stage = [&](int cz, int slot) {
-    const bool zin = cz >= 0 && cz < d.sext[2];
-    int t = 0, yy = warp;
-    for (int r = warp; r < nrows; r += NWARPS, yy += NWARPS) {
-      while (yy >= ncy) { yy -= ncy; ++t; }
-      if (lane < ncx) {
-        const int gy = cy0 + yy;
-        double *sp = coarse + ((slot * NTL + t) * G::CY + yy) * G::CXP + lane;
-        if (zin && xin && gy >= 0 && gy < d.sext[1])
-          cp_async8(sp, d.src[t] + gx + gy * d.ssy + (long long)cz * d.ssz);
-        else
-          *sp = 0.0; // never read by a valid output (host checks the stencils)
-      }
-    }
-  };
-
-  // --- x pass: one coarse base per lane (both its fine points, the copy at
-  // 2c and the interpolant at 2c+1), two rows per warp; x-pass rows are
-  // indexed by fine position minus 2*c_first
-  const int ci = lane & 15, half = lane >> 4;
-  const bool cv = ci <= c_last - c_first;
-  auto xpass = [&](int slot, double *__restrict__ xr) {
-    constexpr int RP = (NTL * G::CY + 1) / 2;      // row pairs, upper bound
-    constexpr int RQ = (RP + NWARPS - 1) / NWARPS; // row pairs per warp
-    const double *__restrict__ cs = coarse;
-#pragma unroll
-    for (int q = 0; q < RQ; ++q) {
-      const int r = 2 * (warp + NWARPS * q) + half;
-      if (r < nrows && cv) {
-        const int t = (r >= ncy) + (NTL > 2 && r >= 2 * ncy);
-        const int yy = r - t * ncy;
-        const double *row = cs + ((slot * NTL + t) * G::CY + yy) * G::CXP + (ci - LO);
-        auto get = [&](int m) { return row[m]; };
-        const double xe = F::template first<FMA>(0, get);
-        const double xo = F::template first<FMA>(1, get);
-        *reinterpret_cast<double2 *>(xr + (t * G::CY + yy) * G::XR + 2 * ci) = make_double2(xe, xo);
-      }
-    }
-  };
-
-  // --- y/z owner: thread = (fine x, coarse y row), both fine y parities
-  const int my_fx = tid % ptx, my_cyr = tid / ptx;
-  const int my_cy = (sy0 >> 1) + my_cyr;
-  const int ys0 = 2 * my_cy, ys1 = ys0 + 1;
-  const bool act = my_cyr < ptyc && my_fx < nfx;
-  const bool v0 = act && ys0 >= sy0 && ys0 < sy0 + nfy;
-  const bool v1 = act && ys1 >= sy0 && ys1 < sy0 + nfy;
-  const int yrow = my_cy - cy0; // index of coarse row my_cy in the plane
-  double *out = d.dst + (d.doff[0] + fx0 + my_fx) + (long long)(d.doff[1] + fy0) * d.dsy +
-                (long long)(d.doff[2] + fz0) * d.dsz;
-
-  // z window: yq[t][h][s] holds the y-pass result of plane p in slot p % Q
-  double yq[NTL][2][Q];
-#pragma unroll
-  for (int t = 0; t < NTL; ++t)
-#pragma unroll
-    for (int h = 0; h < 2; ++h)
-#pragma unroll
-      for (int q = 0; q < Q; ++q) yq[t][h][q] = 0.0;
-
-  // y pass of plane p (slot U = p % Q, static) from its x-pass rows, then
-  // the z outputs whose window plane p completes: coarse base cb = cz - HI,
-  // window planes p-W .. p in slots (U+1+k) % Q
-  auto yzpass = [&](auto Ut, int p, const double *__restrict__ xr) {
-    constexpr int U = decltype(Ut)::value;
-    if (v0 || v1) {
-#pragma unroll
-      for (int t = 0; t < NTL; ++t) {
-        const double *col = xr + (t * G::CY + yrow) * G::XR + my_fx + xoff;
-        auto get = [&](int m) { return col[m * G::XR]; };
-        yq[t][0][U] = F::template next<FMA>(0, get);
-        yq[t][1][U] = F::template next<FMA>(1, get);
-      }
-    }
-    const int cb = cz0 + p - HI;
-#pragma unroll
-    for (int zp = 0; zp < 2; ++zp) {
-      const int zs = 2 * cb + zp;
-      if (zs < sz0 || zs >= sz0 + nfz) continue;
-      double *o = out + (long long)(zs - sz0) * d.dsz;
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        if (!(h ? v1 : v0)) continue;
-        double v[NTL];
-#pragma unroll
-        for (int t = 0; t < NTL; ++t)
-          v[t] = F::template next<FMA>(zp, [&](int m) { return yq[t][h][(U + 1 + (m - LO)) % Q]; });
-        o[(long long)((h ? ys1 : ys0) - sy0) * d.dsy] = tcombine<FMA, TK, NTL>(d.w, v);
-      }
-    }
-  };
-
-  // Pipeline, one barrier per plane: iteration i stages plane i+PD, runs
-  // the x pass of plane i into x-pass buffer i%2 and the y/z passes of plane
-  // i-1 from buffer (i-1)%2.  The staging ring has PD+2 slots, so the slot
-  // being refilled was last read two iterations ago.  The loop is unrolled
-  // by Q so that every z-window slot index is a compile-time constant.
-  const int nplanes = cz1 - cz0 + 1;
-#pragma unroll
-  for (int p = 0; p < G::PD; ++p) {
-    if (p < nplanes) stage(cz0 + p, p);
-    cp_async_commit();
-  }
-  auto iteration = [&](auto Ut, int i) {
-    // Ut: the static value of (i - 1) % Q
-    if (i + G::PD < nplanes) stage(cz0 + i + G::PD, (i + G::PD) % G::NB);
-    cp_async_commit();
-    cp_async_wait<G::PD>();
-    __syncthreads();
-    if (i < nplanes) xpass(i % G::NB, xrows + (i & 1) * S::xbuf);
-    if (i >= 1) yzpass(Ut, i - 1, xrows + ((i - 1) & 1) * S::xbuf);
-  };
-  iteration(std::integral_constant<int, Q - 1>(), 0); // i = 0: x pass only
-  for (int i0 = 1; i0 <= nplanes; i0 += Q) {
-    static_for<Q>([&](auto Ut) {
-      constexpr int u = decltype(Ut)::value;
-      const int i = i0 + u;
-      if (i <= nplanes) iteration(std::integral_constant<int, u>(), i);
-    });
-  }
-  cp_async_wait<0>();
-  __syncthreads(); // shared memory free for the next tile
-  (void)W;
 }
 
 } // namespace cgx

@@ -56,10 +56,10 @@ int launch_map_concurrent(int fp, const Desc *d, const CUtensorMap *maps, const 
                           int nside, int *need, const int *caps = nullptr);
 constexpr int CONCURRENT_SIDE_MAX = NSEG;
 
-// The tensor maps of a prolongation descriptor's source timelevels (cgx.cu):
-// true when the arrays can be staged by TMA (then maps[0 .. ntl-1] are
-// set), false otherwise.
-bool encode_tma_maps(const Desc &d, CUtensorMap maps[3]);
+// The tensor maps of a tiled prolongation descriptor's source timelevels
+// (cgx.cu): true when the arrays can be staged by TMA (then maps[0 .. ntl-1]
+// and d.tma are set), false otherwise.
+bool encode_tma_maps(Desc &d, CUtensorMap maps[3]);
 // tiles of a prolongation descriptor in TMA tile configuration `config`
 long long tile_prolongation(Desc &d, int config);
 
@@ -88,10 +88,9 @@ int klaunch_spair_f1(const Desc &d, int ntiles, int *status, cudaStream_t s);
   int klaunch_tma_f##F##_p##P##_c##C(int variant, const Desc *d, const CUtensorMap *maps,             \
                                      const int2 *tmap, long long ntiles, unsigned long long *counter, \
                                      int *status, cudaStream_t s);
-#define CGX_TMA_DECL5(F, P) \
-  CGX_TMA_DECL(F, P, 0) CGX_TMA_DECL(F, P, 1) CGX_TMA_DECL(F, P, 2) CGX_TMA_DECL(F, P, 3) CGX_TMA_DECL(F, P, 4)
-CGX_TMA_DECL5(0, 0) CGX_TMA_DECL5(0, 1) CGX_TMA_DECL5(1, 0) CGX_TMA_DECL5(1, 1)
-#undef CGX_TMA_DECL5
+#define CGX_TMA_DECL4(F, P) CGX_TMA_DECL(F, P, 0) CGX_TMA_DECL(F, P, 1) CGX_TMA_DECL(F, P, 3) CGX_TMA_DECL(F, P, 4)
+CGX_TMA_DECL4(0, 0) CGX_TMA_DECL4(0, 1) CGX_TMA_DECL4(1, 0) CGX_TMA_DECL4(1, 1)
+#undef CGX_TMA_DECL4
 #undef CGX_TMA_DECL
 int klaunch_stream_f0(int variant, const Desc *d, const int2 *tmap, long long ntiles,
                       unsigned long long *counter, int *status, cudaStream_t s);
@@ -106,7 +105,7 @@ inline bool is_stencil(int kind) {
 }
 inline int segment_of(const Desc &d) {
   if (!is_stencil(d.kind)) return SEG_STREAM + stream_variant(d);
-  const int v = d.bx ? tma_variant(d) : -1;
+  const int v = d.tma ? tma_variant(d) : -1;
   return v >= 0 ? v : SEG_STENCIL;
 }
 

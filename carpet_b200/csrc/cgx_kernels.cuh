@@ -19,23 +19,39 @@
 namespace cgx {
 namespace kern {
 
+// tile configuration of the kernels that stage by cp.async
+static_assert(TMA_CFGS[PLAIN_CFG].nt == NTHREADS, "the cp.async kernels' tiles use every thread");
+
 __device__ __forceinline__ void report(int *status, int code) {
   if (status) atomicCAS(status, 0, code);
 }
 
-// dynamic shared memory of the largest variant a kernel dispatches
-template <int MAXORDER> constexpr int smem_doubles() {
-  return PSmem<VC<MAXORDER>, 3>::total > PSmem<CC<5>, 3>::total
-             ? PSmem<VC<MAXORDER>, 3>::total
-             : PSmem<CC<5>, 3>::total;
+// dynamic shared memory (doubles) of the largest variant a kernel dispatches
+template <class F, int CFG> constexpr int smem_family() {
+  const int a = TSmem<F, 1, CFG>::total, b = TSmem<F, 2, CFG>::total, c = TSmem<F, 3, CFG>::total;
+  return a > b ? (a > c ? a : c) : (b > c ? b : c);
+}
+template <class F, class... R, int CFG> constexpr int smem_max(std::integral_constant<int, CFG> cfg) {
+  const int a = smem_family<F, CFG>();
+  if constexpr (sizeof...(R) == 0) return a;
+  else {
+    const int b = smem_max<R...>(cfg);
+    return a > b ? a : b;
+  }
+}
+template <int CFG, bool HIGH> constexpr int smem_doubles() {
+  if (HIGH) return smem_max<VC<7>, VC<9>, VC<11>>(std::integral_constant<int, CFG>());
+  return smem_max<VC<1>, VC<3>, VC<5>, CC<0>, CC<1>, CC<2>, CC<3>, CC<4>, CC<5>, ENO, CCENO<2>, CCENO<3>>(
+      std::integral_constant<int, CFG>());
 }
 
 // Every tile routine is its own non-inlined function, so that each variant
 // gets its own register allocation instead of sharing one across the whole
 // dispatch switch.  The descriptor is always in shared memory.
-template <class F, int FMA, int NTL, int TK>
+template <class F, int FMA, int NTL, int TK, int CFG>
 __device__ __noinline__ void prolong_entry(const Desc &d, int tile, double *sm) {
-  prolong_tile<F, FMA, NTL, TK>(d, tile, sm);
+  TmaRing none;
+  prolong_tile<F, FMA, NTL, TK, CFG, false>(d, nullptr, tile, sm, none, nullptr);
 }
 template <int FMA, int NTL, int TK>
 __device__ __noinline__ void copy_entry(const Desc &d, int tile) {
@@ -57,22 +73,61 @@ template <int FMA> __device__ __noinline__ void mono_entry(const Desc &d, int ti
   mono_tile<FMA, NTHREADS>(d, tile, threadIdx.x);
 }
 
-template <class F, int FMA>
+template <class F, int FMA, int CFG>
 __device__ __forceinline__ void prolong_ntl(const Desc &d, int tile, double *sm) {
   switch (d.ntl) {
-  case 1: prolong_entry<F, FMA, 1, T_NONE>(d, tile, sm); break;
-  case 2: prolong_entry<F, FMA, 2, T_LIN>(d, tile, sm); break;
+  case 1: prolong_entry<F, FMA, 1, T_NONE, CFG>(d, tile, sm); break;
+  case 2: prolong_entry<F, FMA, 2, T_LIN, CFG>(d, tile, sm); break;
   default:
-    if (d.tkind == T_ENO) prolong_entry<F, FMA, 3, T_ENO>(d, tile, sm);
-    else prolong_entry<F, FMA, 3, T_QUAD>(d, tile, sm);
+    if (d.tkind == T_ENO) prolong_entry<F, FMA, 3, T_ENO, CFG>(d, tile, sm);
+    else prolong_entry<F, FMA, 3, T_QUAD, CFG>(d, tile, sm);
   }
 }
 
-// HIGH selects the vertex-centred orders 7/9/11, which live in their own
-// kernel so that their larger register windows do not lower the occupancy
-// of the common orders.
-template <int FMA, bool HIGH>
-__device__ __forceinline__ void run_tile(const Desc &d, int tile, double *sm, int *status) {
+// The prolongation tiles staged by cp.async, in tile configuration CFG.  HIGH
+// selects the vertex-centred orders 7/9/11, which live in their own kernel so
+// that their longer lines do not lower the occupancy of the common orders.
+template <int FMA, bool HIGH, int CFG>
+__device__ __forceinline__ bool run_prolong(const Desc &d, int tile, double *sm) {
+  if constexpr (HIGH) {
+    if (d.kind != K_PROLONG_VC) return false;
+    switch (d.order) {
+    case 7: prolong_ntl<VC<7>, FMA, CFG>(d, tile, sm); return true;
+    case 9: prolong_ntl<VC<9>, FMA, CFG>(d, tile, sm); return true;
+    case 11: prolong_ntl<VC<11>, FMA, CFG>(d, tile, sm); return true;
+    }
+    return false;
+  } else {
+    switch (d.kind) {
+    case K_PROLONG_VC:
+      switch (d.order) {
+      case 1: prolong_ntl<VC<1>, FMA, CFG>(d, tile, sm); return true;
+      case 3: prolong_ntl<VC<3>, FMA, CFG>(d, tile, sm); return true;
+      case 5: prolong_ntl<VC<5>, FMA, CFG>(d, tile, sm); return true;
+      }
+      return false;
+    case K_PROLONG_CC_ENO:
+      if (d.order == 2) { prolong_ntl<CCENO<2>, FMA, CFG>(d, tile, sm); return true; }
+      if (d.order == 3) { prolong_ntl<CCENO<3>, FMA, CFG>(d, tile, sm); return true; }
+      return false;
+    case K_PROLONG_CC:
+      switch (d.order) {
+      case 0: prolong_ntl<CC<0>, FMA, CFG>(d, tile, sm); return true;
+      case 1: prolong_ntl<CC<1>, FMA, CFG>(d, tile, sm); return true;
+      case 2: prolong_ntl<CC<2>, FMA, CFG>(d, tile, sm); return true;
+      case 3: prolong_ntl<CC<3>, FMA, CFG>(d, tile, sm); return true;
+      case 4: prolong_ntl<CC<4>, FMA, CFG>(d, tile, sm); return true;
+      case 5: prolong_ntl<CC<5>, FMA, CFG>(d, tile, sm); return true;
+      }
+      return false;
+    case K_PROLONG_ENO: prolong_ntl<ENO, FMA, CFG>(d, tile, sm); return true;
+    }
+    return false;
+  }
+}
+
+// every kind of tile, NTHREADS threads (prolongation: configuration 0)
+template <int FMA> __device__ __forceinline__ void run_tile(const Desc &d, int tile, double *sm, int *status) {
   switch (d.kind) {
   case K_COPY:
     if (d.ntl == 1) copy_entry<FMA, 1, T_NONE>(d, tile);
@@ -85,54 +140,18 @@ __device__ __forceinline__ void run_tile(const Desc &d, int tile, double *sm, in
   case K_RESTRICT_CC3: restrict_cc3_entry<FMA>(d, tile); return;
   case K_RESTRICT_CC5: restrict_cc5_entry<FMA>(d, tile); return;
   case K_PROLONG_MONO: mono_entry<FMA>(d, tile); return;
-  case K_PROLONG_VC:
-    if (HIGH) {
-      switch (d.order) {
-      case 7: prolong_ntl<VC<7>, FMA>(d, tile, sm); return;
-      case 9: prolong_ntl<VC<9>, FMA>(d, tile, sm); return;
-      case 11: prolong_ntl<VC<11>, FMA>(d, tile, sm); return;
-      }
-    } else {
-      switch (d.order) {
-      case 1: prolong_ntl<VC<1>, FMA>(d, tile, sm); return;
-      case 3: prolong_ntl<VC<3>, FMA>(d, tile, sm); return;
-      case 5: prolong_ntl<VC<5>, FMA>(d, tile, sm); return;
-      }
-    }
-    break;
-  case K_PROLONG_CC_ENO:
-    if (!HIGH) {
-      if (d.order == 2) { prolong_ntl<CCENO<2>, FMA>(d, tile, sm); return; }
-      if (d.order == 3) { prolong_ntl<CCENO<3>, FMA>(d, tile, sm); return; }
-    }
-    break;
-  case K_PROLONG_CC:
-    if (!HIGH) {
-      switch (d.order) {
-      case 0: prolong_ntl<CC<0>, FMA>(d, tile, sm); return;
-      case 1: prolong_ntl<CC<1>, FMA>(d, tile, sm); return;
-      case 2: prolong_ntl<CC<2>, FMA>(d, tile, sm); return;
-      case 3: prolong_ntl<CC<3>, FMA>(d, tile, sm); return;
-      case 4: prolong_ntl<CC<4>, FMA>(d, tile, sm); return;
-      case 5: prolong_ntl<CC<5>, FMA>(d, tile, sm); return;
-      }
-    }
-    break;
-  case K_PROLONG_ENO:
-    if (!HIGH) { prolong_ntl<ENO, FMA>(d, tile, sm); return; }
-    break;
   }
-  if (threadIdx.x == 0) report(status, CGX_EDEVICE);
+  if (!run_prolong<FMA, false, PLAIN_CFG>(d, tile, sm) && threadIdx.x == 0) report(status, CGX_EDEVICE);
 }
 
 template <int FMA, bool HIGH>
-__global__ void __launch_bounds__(NTHREADS, 2)
+__global__ void __launch_bounds__(NTHREADS, HIGH ? 1 : 2)
     k_pair(const __grid_constant__ Desc d, int *status) {
   extern __shared__ __align__(16) double sm[];
   __shared__ __align__(16) Desc s_d;
   if (threadIdx.x == 0) s_d = d; // field-wise copy out of the parameter space
   __syncthreads();
-  run_tile<FMA, HIGH>(s_d, blockIdx.x, sm, status);
+  if (!run_prolong<FMA, HIGH, PLAIN_CFG>(s_d, blockIdx.x, sm) && threadIdx.x == 0) report(status, CGX_EDEVICE);
 }
 
 // Persistent form: each CTA repeatedly claims the next tile index from
@@ -170,7 +189,7 @@ __global__ void __launch_bounds__(NTHREADS, 2)
       reinterpret_cast<unsigned long long *>(&s_d)[threadIdx.x] =
           __ldg(reinterpret_cast<const unsigned long long *>(descs + di) + threadIdx.x);
     __syncthreads();
-    run_tile<FMA, false>(s_d, (int)(t - prefix[di]), sm, status);
+    run_tile<FMA>(s_d, (int)(t - prefix[di]), sm, status);
     __syncthreads(); // s_tile, s_desc and s_d are free for the next claim
   }
 }
@@ -228,7 +247,7 @@ __global__ void __launch_bounds__(NTHREADS, 2)
     unsigned long long tn = 0;
     if (threadIdx.x == 0) tn = atomicAdd(counter, 1ULL);
     __syncthreads();
-    run_tile<FMA, false>(s_d, m.y, sm, status);
+    if (!run_prolong<FMA, false, PLAIN_CFG>(s_d, m.y, sm) && threadIdx.x == 0) report(status, CGX_EDEVICE);
     __syncthreads(); // everyone is done with s_d, s_t and s_m
     if (threadIdx.x == 0) {
       s_t = (long long)tn;
@@ -337,10 +356,10 @@ __global__ void __launch_bounds__(STREAM_THREADS, STREAM_MAP_BLOCKS_PER_SM)
 // ---------------------------------------------------------------- TMA form
 // One persistent kernel per prolongation variant (family, order, time
 // interpolation), so that each gets its own register allocation; maps[3 * i
-// + t] is the tensor map of descriptor i's timelevel t.  The claim loop is
-// that of k_stream_map.
+// + t] is the tensor map of descriptor i's timelevel t.  Thread 0 claims the
+// next tile while the current one runs.
 template <int FMA, class F, int NTL, int TK, int CFG>
-__global__ void __launch_bounds__(TMA_CFGS[CFG].nt, TMA_CFGS[CFG].mb)
+__global__ void __launch_bounds__(TMA_CFGS[CFG].nt, tma_blocks<F, NTL, TK, CFG>())
     k_tma_map(const Desc *__restrict__ descs, const CUtensorMap *__restrict__ maps,
               const int2 *__restrict__ tmap, long long ntiles, unsigned long long *counter, int *status,
               int variant) {
@@ -352,22 +371,19 @@ __global__ void __launch_bounds__(TMA_CFGS[CFG].nt, TMA_CFGS[CFG].mb)
   __shared__ long long s_t, s_next;
   __shared__ int2 s_m;
   __shared__ __align__(16) Desc s_d;
-  __shared__ __align__(8) uint64_t s_bars[TMA_NB_MAX];
-  __shared__ int s_abort;
+  __shared__ __align__(8) uint64_t s_bars[TMA_NB];
   // bit 30 of variant: failure injection (cgx_debug_skip_tma_plane)
-  const int skip = (variant >> 30) & 1 ? 0 : -1;
+  TmaRing ring{s_bars, 0u, ((variant >> 30) & 1) != 0};
   variant &= ~(1 << 30);
   pdl_wait();
   if (threadIdx.x == 0) {
-    for (int i = 0; i < TMA_NB_MAX; ++i) mbar_init(&s_bars[i], 1);
+    for (int i = 0; i < TMA_NB; ++i) mbar_init(&s_bars[i], 1);
     mbar_fence_init();
-    s_abort = 0;
     const long long t = (long long)atomicAdd(counter, 1ULL);
     s_t = t;
     s_m = t < ntiles ? tmap[t] : make_int2(0, 0);
   }
   __syncthreads();
-  TmaRing ring{s_bars, &s_abort, 0u, skip};
   for (;;) {
     if (s_t >= ntiles) {
       if (threadIdx.x == 0) claims_done(counter);
@@ -381,14 +397,13 @@ __global__ void __launch_bounds__(TMA_CFGS[CFG].nt, TMA_CFGS[CFG].mb)
     __syncthreads();
     if (s_next >= ntiles) pdl_trigger(); // this CTA's last tile
     if (tma_variant(s_d) == variant) {
-      if (!prolong_tile_tma<F, FMA, NTL, TK, CFG>(s_d, maps + 3 * (size_t)m.x, m.y, sm, ring, status)) {
+      if (!prolong_tile<F, FMA, NTL, TK, CFG, true>(s_d, maps + 3 * (size_t)m.x, m.y, sm, ring, status)) {
         if (threadIdx.x == 0) claims_done(counter);
         return;
       }
     } else if (threadIdx.x == 0) {
       report(status, CGX_EDEVICE);
     }
-    __syncthreads();
     if (threadIdx.x == 0) {
       const long long tn = s_next;
       s_t = tn;
@@ -400,7 +415,7 @@ __global__ void __launch_bounds__(TMA_CFGS[CFG].nt, TMA_CFGS[CFG].mb)
 
 // dynamic shared memory of the widest variant a kernel dispatches
 inline size_t smem_bytes(bool high) {
-  return sizeof(double) * (high ? smem_doubles<11>() : smem_doubles<5>());
+  return sizeof(double) * (high ? smem_doubles<PLAIN_CFG, true>() : smem_doubles<PLAIN_CFG, false>());
 }
 
 } // namespace kern

@@ -541,7 +541,7 @@ int cgx_server_define_op(cgx_server *sv, int hier, const cgx_batch *pairs, int *
       pd[i] = t;
       pnt[i] = tn;
     } else {
-      pd[i].bx = 0;
+      pd[i].tma = 0;
     }
   }
   for (int i = 0; i < n; ++i) {

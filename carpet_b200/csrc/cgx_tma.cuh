@@ -1,23 +1,35 @@
-// cgx_tma.cuh -- prolongation with TMA staging (device code).
+// cgx_tma.cuh -- prolongation tiles (device code).
 //
-// The same separable x -> y -> z arithmetic as prolong_tile (cgx_device.cuh),
-// organised so that every thread's work is fixed per tile and the plane loop
-// is straight-line code:
+// Separable x -> y -> z passes over a tile, the time interpolation fused, in
+// CarpetLib's operation order.  A CTA marches its tile in stages of bz coarse
+// planes:
 //
-//   * one elected thread stages each coarse plane with one bulk tensor copy
-//     per timelevel (cp.async.bulk.tensor, a box of bx x by coarse points),
-//     completing on an mbarrier per ring slot; boxes may start outside the
-//     array (zero fill), which only masked outputs read;
-//   * the x pass is a flat list of (timelevel, coarse row, coarse base)
-//     items spread over all threads, whatever the tile's shape; each item's
-//     shared-memory offsets are computed once per tile;
-//   * the y/z pass keeps its thread = (fine x, coarse y row) mapping and
-//     register z window; threads without a point compute on clamped
-//     indices and their stores are masked, so no branch diverges.
+//   * staging: the stage's coarse box (bx points, by rows, bz planes, every
+//     timelevel) lies in one of two shared-memory slots.  TMA form: one
+//     elected thread issues one bulk tensor copy per timelevel
+//     (cp.async.bulk.tensor), completing on the slot's mbarrier; boxes may
+//     start outside the array (zero fill), which only masked outputs read.
+//     Plain form (arrays the tensor-copy unit cannot address): cp.async by
+//     all threads.  The copies of stage s + 2 start once the x pass has read
+//     stage s, and have the y/z pass of a whole stage to land;
+//   * x pass: one thread per (timelevel, plane, coarse row) walks its row
+//     (Line), two points per 16-byte load: by rows of an odd number of
+//     16-byte units, so that the lanes of a quarter warp, which hold
+//     consecutive rows, meet no bank conflict.  One item per (row, base), as
+//     a window form would have it, loads 6 points per base instead of 1.6
+//     and spent half of the kernel's shared-memory wavefronts;
+//   * y/z pass: thread = (fine x, coarse y row) takes the window of its row
+//     from the x-pass rows, both fine y, and pushes them into its z lines,
+//     whose open sums stay in registers over the whole tile; threads without
+//     a point compute on clamped indices and their stores are masked, so no
+//     branch diverges.
 //
-// A descriptor is eligible when its source arrays can be described to the
-// tensor-copy unit (16-byte aligned base, even row and plane pitches); the
-// host builds one CUtensorMap per timelevel at upload time.
+// Two barriers per stage.  What bounds it: instruction issue and the FP64
+// pipe (the exact mode's separate products and sums), not DRAM.
+//
+// A descriptor is staged by TMA when its source arrays can be described to
+// the tensor-copy unit (16-byte aligned base, even row and plane pitches);
+// the host builds one CUtensorMap per timelevel.
 #pragma once
 #include <cuda.h>
 
@@ -26,50 +38,77 @@
 namespace cgx {
 
 // Tile configurations the autotuner chooses between: threads per CTA, coarse
-// y rows per tile (threads / 16: one thread per fine x and coarse row), fine
-// z points per tile, CTAs per SM the register allocation must allow, and
-// planes staged ahead of the x pass.  Configuration 0 is the default.
+// y rows of a 16-wide tile (threads / 16: one thread per fine x and coarse
+// row), the most fine z points per tile, CTAs per SM the register allocation
+// must allow.  Configuration 0 is the default.  Configurations that differ
+// in pz alone share their kernels (tma_kernel_cfg).  mb is that of the widest
+// common case, order 5 with three timelevels (tma_blocks).
 struct TmaCfg {
-  int nt, pyc, pz, mb, pd;
+  int nt, pyc, pz, mb;
 };
-constexpr TmaCfg TMA_CFGS[] = {
-    {256, 16, 64, 2, 3}, {128, 8, 64, 4, 3}, {128, 8, 32, 4, 3}, {128, 8, 64, 5, 2}, {128, 8, 32, 6, 2}};
+constexpr TmaCfg TMA_CFGS[] = {{256, 16, 64, 2}, {128, 8, 64, 4}, {128, 8, 32, 4}, {128, 8, 64, 5}, {128, 8, 32, 6}};
 constexpr int TMA_NCFG = 5;
-constexpr int TMA_NB_MAX = 5; // ring slots, at most (pd + 2)
+constexpr int tma_kernel_cfg(int c) { return c == 2 ? 1 : c; }
+// the configuration of the kernels that stage by cp.async
+constexpr int PLAIN_CFG = 0;
+// mbarriers per CTA: one per stage slot
+constexpr int TMA_NB = 2;
 
-// Shared-memory geometry of a tile configuration with PYC coarse rows for a
-// stencil window of width W (host and device).  A tile of ptx fine x uses
-// ptx * ptyc owner threads; ptyc may exceed PYC when ptx < 16, as far as the
-// staged box, the x-pass rows and the x items fit (tma_rows_max, host).
-//   coarse box      bx = (ptx + 2) / 2 bases + the window + one point of
-//                   even-alignment shift, rounded up to even; by = ptyc + W
-//                   rows; bx * by <= tma_tls doubles per (slot, timelevel)
-//   x-pass rows     ntl * by rows of pitch TMA_XR (two fine points per coarse
-//                   base: at most ptx + 2 <= 18), + one spare row for masked
-//                   x items; a half-warp of the y pass reads one row when
-//                   ptx = 16, at most three short rows otherwise
-//   x items         (timelevel, coarse row, coarse base), at most
-//                   ntl * tma_items per tile
-constexpr int TMA_EXTRA_ROWS = 3; // rows staged beyond PYC + W (for ptx < 16)
-__host__ __device__ constexpr int tma_bxmax(int W) { return ((PTXMAX + 2) / 2 + W + 2) & ~1; }
-__host__ __device__ constexpr int tma_bymax(int W, int pyc) { return pyc + W + TMA_EXTRA_ROWS; }
-__host__ __device__ constexpr int tma_tls(int W, int pyc) { return (tma_bxmax(W) * tma_bymax(W, pyc) + 15) / 16 * 16; }
+// Shared-memory geometry of a tile configuration for a stencil window of
+// width W and NTL timelevels (host and device).
+//   stage      bx = the coarse bases + the window + one point of
+//              even-alignment shift, rounded up to an odd number of 16-byte
+//              units; by = ptyc + W rows; bz planes; by * bz <= tma_rpt and
+//              bx * by * bz <= tma_tls per (slot, timelevel)
+//   x-pass rows  one per (timelevel, plane, row), pitch TMA_XR (two fine
+//              points per coarse base, at most 9 bases): NTL * by * bz <= NT,
+//              one thread each
+// tma_rpt is sized for whole planes of pyc + 1 rows: three planes of three
+// timelevels in 128 threads.  TMA_PMAX planes at most: more planes per stage
+// mean fewer barriers, but less room for other CTAs.
 constexpr int TMA_XR = PTXMAX + 2; // even: 16-byte rows
-__host__ __device__ constexpr int tma_xbuf(int W, int pyc, int ntl) { return (ntl * tma_bymax(W, pyc) + 1) * TMA_XR; }
-__host__ __device__ constexpr int tma_items(int W, int pyc) { return (pyc + W) * ((PTXMAX + 2) / 2); }
+constexpr int TMA_PMAX = 4;
+__host__ __device__ constexpr int tma_bx(int nbx, int W) {
+  const int e = (nbx + W + 2) & ~1;
+  return e / 2 % 2 ? e : e + 2;
+}
+__host__ __device__ constexpr int tma_rpt(int W, int nt, int pyc, int ntl, int planes) {
+  const int by = pyc + W + 1, p = nt / (ntl * by);
+  const int q = planes ? planes : p < 1 ? 1 : p > TMA_PMAX ? TMA_PMAX : p;
+  return q * by < nt / ntl ? q * by : nt / ntl;
+}
+__host__ __device__ constexpr int tma_tls(int W, int nt, int pyc, int ntl, int planes) {
+  return (tma_bx(PTXMAX / 2, W) * tma_rpt(W, nt, pyc, ntl, planes) + 15) / 16 * 16;
+}
 
-template <class F, int PYC = PTYCMAX> struct TGeom {
+// Planes per stage of the one-timelevel tiles: whole turns of the phases of a
+// family's z lines, so that every plane of a stage has its phase at compile
+// time; 0 where the phase is carried (three timelevels: a turn of order 5
+// would take 195 threads and half of the shared memory again).
+__host__ __device__ constexpr int tma_planes(int phases, int ntl) { return ntl == 1 ? (3 + phases) / phases * phases : 0; }
+
+template <class F, int NTL, int CFG> struct TSmem {
   static constexpr int W = F::HI - F::LO;
-  static constexpr int TLS = tma_tls(W, PYC); // doubles per (slot, timelevel)
-  static constexpr int ITEMS = tma_items(W, PYC);
-  static constexpr int Q = W + 1;
+  static constexpr int NT = TMA_CFGS[CFG].nt, PYC = TMA_CFGS[CFG].pyc;
+  static constexpr int P = tma_planes(F::PHASES, NTL);
+  static constexpr int RPT = tma_rpt(W, NT, PYC, NTL, P); // rows per (slot, timelevel)
+  static constexpr int TLS = tma_tls(W, NT, PYC, NTL, P); // doubles per (slot, timelevel)
+  static constexpr int coarse = TMA_NB * NTL * TLS;
+  static constexpr int total = coarse + NTL * RPT * TMA_XR; // doubles
+  static_assert(NTL * RPT <= NT, "one thread per x-pass row");
 };
-template <class F, int NTL, int PYC = PTYCMAX, int NB = 5> struct TSmem {
-  using G = TGeom<F, PYC>;
-  static constexpr int coarse = NB * NTL * G::TLS;
-  static constexpr int xbuf = tma_xbuf(G::W, PYC, NTL);
-  static constexpr int total = coarse + 2 * xbuf; // doubles
-};
+
+// CTAs per SM that a variant's register allocation must allow: what its open
+// z sums (two lines per timelevel) and about 48 other registers leave room
+// for, and as many more as the configuration asks beyond that case's 4 of 128
+// threads.
+template <class F, int NTL, int TK, int CFG> constexpr int tma_blocks() {
+  constexpr int line = sizeof(typename F::template Line<0, false>) / 4;
+  constexpr int regs = 2 * NTL * line + 48 + (TK == T_ENO ? 16 : 0);
+  constexpr int NT = TMA_CFGS[CFG].nt, extra = TMA_CFGS[CFG].mb - 512 / NT;
+  constexpr int b = 65536 / (NT * regs) + extra;
+  return b < 1 ? 1 : b > 1024 / NT ? 1024 / NT : b;
+}
 
 // The TMA kernels' variants: family (VC 1/3/5, CC 0-5, ENO) x time
 // interpolation (one timelevel, linear, quadratic, ENO).
@@ -129,271 +168,276 @@ __device__ __forceinline__ void tma_load_3d(double *dst, const CUtensorMap *map,
                : "memory");
 }
 
-// Ring state of one CTA: planes staged so far (plane g uses slot g % NB,
-// whose phase g / NB completes when it lands), and a flag that a wait ran
-// out.  Everything here is uniform over the CTA.
+// Where a tile lies in its region: first fine point and extent.  y and z
+// tiles start at even source positions: the first tile is one point short
+// where the region starts at an odd one, and every tile's coarse rows and
+// planes serve two fine points each.  x0: start of the x tile (d.xo).
+struct TileGeo {
+  int f0[3], n[3], x0;
+};
+__device__ __forceinline__ TileGeo tile_geo(const Desc &d, int tile) {
+  const int rr = (int)div_magic((unsigned)tile, d.mg[0], d.sh[0]), tz = (int)div_magic((unsigned)rr, d.mg[1], d.sh[1]);
+  const int t[3] = {tile - rr * d.tiles[0], rr - tz * d.tiles[1], tz};
+  const int w[3] = {d.xw, 2 * d.ptyc, d.pz}, o[3] = {d.xo, d.soff[1] & 1, d.soff[2] & 1};
+  TileGeo g;
+  g.x0 = t[0] * w[0] - o[0];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    g.f0[k] = max(0, t[k] * w[k] - o[k]);
+    g.n[k] = min((t[k] + 1) * w[k] - o[k] + (k == 0 ? d.xs2 : 0), d.n[k]) - g.f0[k];
+  }
+  return g;
+}
+
+// Staging state of one CTA.  Stages are counted over all its tiles: stage g
+// uses slot g % 2, whose mbarrier phase g / 2 completes when it lands.
 struct TmaRing {
-  uint64_t *bars; // pd + 2 mbarriers, arrival count 1
-  int *abort;     // shared flag, set when a wait gave up
-  unsigned g;     // planes staged by this CTA before the current tile
+  uint64_t *bars = nullptr; // TMA_NB mbarriers, arrival count 1
+  unsigned g = 0;           // stages of the earlier tiles
   // failure injection for the tests of the bounded waits
-  // (cgx_debug_skip_tma_plane): the plane of this CTA's first tile that is
-  // never staged, so that the wait for it runs out; -1 in normal use
-  int skip = -1;
+  // (cgx_debug_skip_tma_plane): stage 0 is never staged, so that the wait for
+  // it runs out
+  bool skip = false;
 };
 
-// One prolongation tile.  Returns false when a wait gave up (the CTA then
-// stops; the status word holds CGX_EDEVICE).
-template <class F, int FMA, int NTL, int TK, int CFG>
-__device__ bool prolong_tile_tma(const Desc &d, const CUtensorMap *__restrict__ maps, int tile, double *sm,
-                                 TmaRing &ring, int *status) {
-  constexpr int NT = TMA_CFGS[CFG].nt, PYC = TMA_CFGS[CFG].pyc, PZ = TMA_CFGS[CFG].pz;
-  constexpr int PD = TMA_CFGS[CFG].pd, NB = PD + 2;
-  using G = TGeom<F, PYC>;
-  using S = TSmem<F, NTL, PYC, NB>;
-  constexpr int LO = F::LO, HI = F::HI, Q = G::Q;
-  constexpr bool SPLIT = NTL == 1;
-  const int tid = threadIdx.x;
-  const int ptx = d.ptx, ptyc = d.ptyc, pty = 2 * ptyc - 1;
-  const int BX = d.bx, BY = d.by;
-  // x-pass rows: BY per timelevel, pitch XR
-  constexpr int XR = TMA_XR;
-  const int CY = BY;
-
-  const int tx = tile % d.tiles[0], rr = tile / d.tiles[0];
-  const int ty = rr % d.tiles[1], tz = rr / d.tiles[1];
-  const int fx0 = tx * ptx, fy0 = ty * pty, fz0 = tz * PZ;
-  const int nfx = min(ptx, d.n[0] - fx0), nfy = min(pty, d.n[1] - fy0), nfz = min(PZ, d.n[2] - fz0);
-  const int sx0 = d.soff[0] + fx0, sy0 = d.soff[1] + fy0, sz0 = d.soff[2] + fz0;
-  const int c_first = sx0 >> 1, c_last = (sx0 + nfx - 1) >> 1;
-  const int cx0 = c_first + LO;
-  const int bx0 = cx0 & ~1; // box start: an even x coordinate
-  const int xs = cx0 - bx0;
-  const int cy0 = (sy0 >> 1) + LO, cy1 = ((sy0 + nfy - 1) >> 1) + HI;
-  const int cz0 = (sz0 >> 1) + LO, cz1 = ((sz0 + nfz - 1) >> 1) + HI;
-  const int nbx = c_last - c_first + 1, ncy = cy1 - cy0 + 1;
-  const int nplanes = cz1 - cz0 + 1;
-  const int xoff = sx0 - 2 * c_first;
-  const unsigned g0 = ring.g;
-
-  double *coarse = sm;
-  double *xrows = sm + S::coarse;
-
-  int issued = 0; // planes staged so far (elected thread)
-  const int skip = g0 == 0 ? ring.skip : -1;
-  int islot = (int)(g0 % NB); // multi-timelevel: ring slot of the next plane staged
-  auto issue = [&](int p) {   // elected thread: stage plane p (p = 0, 1, ...)
-    issued = p + 1;
-    int slot;
-    if constexpr (SPLIT) {
-      slot = (int)((g0 + (unsigned)p) % NB);
-    } else {
-      slot = islot;
-      if (++islot == NB) islot = 0;
+// The x pass over one staged row: src is its first point (16-byte aligned),
+// which lies xs (0 or 1) points before the window of base 0; writes the two
+// fine points of bases 0 .. nbx-1 to dst.  NBX and XS give them as constants
+// (NBX = 0: nbx, xs), which leaves out the sums that no base reads: 80
+// instead of 120 operations for 8 bases of order 5.
+template <class F, int FMA, int NBX, int XS>
+__device__ __forceinline__ void x_line(const double *__restrict__ src, double *__restrict__ dst, int xs, int nbx) {
+  constexpr int W = F::HI - F::LO, DD = F::D1 - F::D0;
+  constexpr int QN = NBX ? (XS + NBX + W + 1) / 2 : tma_bx(PTXMAX / 2 + 1, W) / 2;
+  if (NBX) nbx = NBX, xs = XS;
+  typename F::template Line<FMA, true> line;
+  const int nload = xs + nbx + W;
+  double e[2 * QN];
+  static_for<QN>([&](auto Q) {
+    constexpr int q = decltype(Q)::value;
+    if (NBX || 2 * q < nload) { // uniform
+      const double2 v = *reinterpret_cast<const double2 *>(src + 2 * q);
+      static_for<2>([&](auto K) {
+        constexpr int j = 2 * q + decltype(K)::value;
+        constexpr Open w{j, XS, NBX ? XS + NBX : 1 << 30};
+        if (NBX && j >= XS + NBX + W) return;
+        double o1 = 0.0;
+        line.template push<j % F::PHASES>(j & 1 ? v.y : v.x, e[j], o1, w);
+        // completes base j - W - xs
+        if (j >= W && (j > W || xs == 0) && j - W - xs < nbx)
+          *reinterpret_cast<double2 *>(dst + 2 * (j - W - xs)) = make_double2(e[j >= W ? j - DD : 0], o1);
+      });
     }
-    if (p == skip) return; // failure injection: this plane never lands
-    mbar_expect_tx(&ring.bars[slot], (unsigned)(NTL * BX * BY * 8));
-#pragma unroll
-    for (int t = 0; t < NTL; ++t)
-      tma_load_3d(coarse + (slot * NTL + t) * G::TLS, maps + t, &ring.bars[slot], bx0, cy0, cz0 + p);
-  };
-
-  // --- x items: (timelevel, row, base) spread over the CTA
-  constexpr int IT = (NTL * G::ITEMS + NT - 1) / NT; // ncy * nbx <= ITEMS
-  const int per_t = ncy * nbx, count = NTL * per_t;
-  int xsrc[IT], xdst[IT];
-#pragma unroll
-  for (int k = 0; k < IT; ++k) {
-    const int it = tid + k * NT;
-    if (it < count) {
-      const int t = it / per_t, rem = it - t * per_t;
-      const int r = rem / nbx, b = rem - r * nbx;
-      xsrc[k] = t * G::TLS + r * BX + xs + b; // window element j of base b at xsrc + j - LO
-      xdst[k] = (t * CY + r) * XR + 2 * b;
-    } else {
-      xsrc[k] = 0;
-      xdst[k] = NTL * CY * XR; // the spare row
-    }
+  });
+}
+template <class F, int FMA>
+__device__ __forceinline__ void x_row(const double *__restrict__ src, double *__restrict__ dst, int xs, int nbx) {
+  constexpr int FULL = PTXMAX / 2;
+  if (F::PHASES > 1 && nbx == FULL) { // uniform
+    if (xs) x_line<F, FMA, FULL, 1>(src, dst, 1, FULL);
+    else x_line<F, FMA, FULL, 0>(src, dst, 0, FULL);
+  } else {
+    x_line<F, FMA, 0, 0>(src, dst, xs, nbx);
   }
-  auto xpass = [&](int slot, double *__restrict__ xr) {
-    const double *__restrict__ cs = coarse + slot * NTL * G::TLS - LO;
-    // every thread runs its items of all rounds but, without SPLIT, the last
-    // one when the tile has no item there (items past the plane's count read
-    // the slot's first points and write the spare row)
-#pragma unroll
-    for (int k = 0; k < IT; ++k) {
-      if (SPLIT || k < IT - 1 || k * NT < count) { // uniform
-        const double *row = cs + xsrc[k];
-        auto get = [&](int m) { return row[m]; };
-        const double xe = F::template first<FMA>(0, get);
-        const double xo = F::template first<FMA>(1, get);
-        *reinterpret_cast<double2 *>(xr + xdst[k]) = make_double2(xe, xo);
-      }
-    }
+}
+
+// fn(integral_constant<int, phase>()), phase < N uniform over the warp
+template <int N, class Fn> __device__ __forceinline__ void by_phase(int phase, Fn &&fn) {
+  auto one = [&](auto K) {
+    if constexpr ((decltype(K)::value) < N) fn(K);
+    else __builtin_unreachable();
   };
+  static_assert(N <= 11, "a case per phase");
+  switch (phase) {
+  case 0: one(std::integral_constant<int, 0>()); break;
+  case 1: one(std::integral_constant<int, 1>()); break;
+  case 2: one(std::integral_constant<int, 2>()); break;
+  case 3: one(std::integral_constant<int, 3>()); break;
+  case 4: one(std::integral_constant<int, 4>()); break;
+  case 5: one(std::integral_constant<int, 5>()); break;
+  case 6: one(std::integral_constant<int, 6>()); break;
+  case 7: one(std::integral_constant<int, 7>()); break;
+  case 8: one(std::integral_constant<int, 8>()); break;
+  case 9: one(std::integral_constant<int, 9>()); break;
+  case 10: one(std::integral_constant<int, 10>()); break;
+  default: __builtin_unreachable();
+  }
+}
+
+// One prolongation tile.  Returns false when a wait gave up (the CTA then
+// stops; the status word holds CGX_EDEVICE).  TMA: staged by tensor copies
+// (maps, ring), else by cp.async from d.src.
+template <class F, int FMA, int NTL, int TK, int CFG, bool TMA>
+__device__ __forceinline__ bool prolong_tile(const Desc &d, const CUtensorMap *__restrict__ maps, int tile,
+                                             double *sm, TmaRing &ring, int *status) {
+  using S = TSmem<F, NTL, CFG>;
+  constexpr int NT = S::NT, LO = F::LO, HI = F::HI, D0 = F::D0, D1 = F::D1, XR = TMA_XR;
+  constexpr int BZS = tma_planes(F::PHASES, NTL); // planes per stage where fixed
+  const int tid = threadIdx.x;
+  const int BX = d.bx, BY = d.by, BZ = BZS ? BZS : d.bz;
+  const TileGeo geo = tile_geo(d, tile);
+  const int fx0 = geo.f0[0], nfx = geo.n[0], nfy = geo.n[1], nfz = geo.n[2];
+  const int sx0 = d.soff[0] + fx0, sy0 = d.soff[1] + geo.f0[1], sz0 = d.soff[2] + geo.f0[2];
+  const int c_first = sx0 >> 1, nbx = ((sx0 + nfx - 1) >> 1) - c_first + 1;
+  // the staged boxes start at an even x coordinate (the 16-byte rule)
+  const int bx0 = (c_first + LO) & ~1, xs = c_first + LO - bx0;
+  const int cy0 = (sy0 >> 1) + LO, cz0 = (sz0 >> 1) + LO;
+  // planes: up to the last one an output needs (the parity-0 value of the
+  // last point may need one fewer than the parity-1 value)
+  const int zlast = sz0 + nfz - 1;
+  const int nplanes = ((zlast - (D0 < D1 && !(zlast & 1) ? 1 : 0)) >> 1) + HI - cz0 + 1;
+  const int nstages = (nplanes + BZ - 1) / BZ;
+  const int rows = BY * BZ; // x-pass rows per timelevel
+
+  double *const coarse = sm;
+  double *const xrows = sm + S::coarse;
+
+  // --- staging: stage s (s = 0, 1, ...) into slot (g0 + s) % 2
+  const unsigned g0 = ring.g;
+  auto issue = [&](int s) { // TMA form: the elected thread
+    if (ring.skip && g0 == 0 && s == 0) return; // failure injection
+    const unsigned g = g0 + (unsigned)s;
+    double *slot = coarse + (g & 1u) * (NTL * S::TLS);
+    uint64_t *bar = &ring.bars[g & 1u];
+    mbar_expect_tx(bar, (unsigned)(NTL * 8 * BX * rows));
+#pragma unroll
+    for (int t = 0; t < NTL; ++t) tma_load_3d(slot + t * S::TLS, maps + t, bar, bx0, cy0, cz0 + s * BZ);
+  };
+  auto fetch = [&](int s) { // all threads: a warp per row, a lane per point
+    double *slot = coarse + ((g0 + (unsigned)s) & 1u) * (NTL * S::TLS);
+    const int lane = tid & 31, gx = bx0 + lane;
+    if (lane < BX)
+      for (int r = tid >> 5; r < NTL * rows; r += NT / 32) {
+        const int t = (r >= rows) + (NTL > 2 && r >= 2 * rows), q = r - t * rows;
+        const int p = q / BY, gy = cy0 + (q - p * BY), gz = cz0 + s * BZ + p;
+        double *sp = slot + t * S::TLS + q * BX + lane;
+        if (gx >= 0 && gx < d.sext[0] && gy >= 0 && gy < d.sext[1] && gz >= 0 && gz < d.sext[2])
+          cp_async8(sp, d.src[t] + gx + gy * d.ssy + gz * d.ssz);
+        else
+          *sp = 0.0; // never read by a valid output (the host checks the stencils)
+      }
+  };
+  if constexpr (TMA) {
+    if (tid == 0) {
+      issue(0);
+      if (nstages > 1) issue(1);
+    }
+  } else {
+    fetch(0);
+    cp_async_commit();
+    if (nstages > 1) fetch(1);
+    cp_async_commit();
+  }
+
+  // --- x pass: thread = (timelevel, plane, row)
+  const int xt = (tid >= rows) + (NTL > 2 && tid >= 2 * rows); // timelevel, where tid < NTL * rows
+  const double *const xsrc = coarse + xt * S::TLS + (tid - xt * rows) * BX;
+  double *const xdst = xrows + tid * XR;
 
   // --- y/z owner: thread = (fine x, coarse y row) = (tid % ptx, tid / ptx);
   // threads past the ptx * ptyc owners address row ptyc - 1 and store nothing
-  static_assert(PTXMAX == 16 && NT == 16 * PYC, "y/z thread layout of a full-width tile");
-  const int my_fx = tid % ptx, my_cyr_all = tid / ptx;
-  const bool tact = my_cyr_all < ptyc;
-  const int my_cyr = tact ? my_cyr_all : ptyc - 1;
-  const bool wact = (tid & ~31) / ptx < ptyc; // warp holds an owner
-  const int my_cy = (sy0 >> 1) + my_cyr;
-  const int ys0 = 2 * my_cy;
-  const bool xin = tact && my_fx < nfx;
-  const bool v0 = xin && ys0 >= sy0 && ys0 < sy0 + nfy;
-  const bool v1 = xin && ys0 + 1 >= sy0 && ys0 + 1 < sy0 + nfy;
-  const int ycol = (my_cyr - LO) * XR + my_fx + xoff;
+  const int my_cyr_all = (tid * d.rpx) >> 16, my_fx = tid - my_cyr_all * d.ptx;
+  const bool tact = my_cyr_all < d.ptyc;
+  const int my_cyr = tact ? my_cyr_all : d.ptyc - 1;
+  const bool wact = (((tid & ~31) * d.rpx) >> 16) < d.ptyc; // warp holds an owner
+  const int ys0 = 2 * ((sy0 >> 1) + my_cyr);
   const long long dsy = d.dsy, dsz = d.dsz;
-  double *const obase = d.dst + (d.doff[0] + fx0 + my_fx) + (long long)(d.doff[1] + fy0 + ys0 - sy0) * dsy +
-                        (long long)(d.doff[2] + fz0 - sz0) * dsz;
+  int zs = 2 * (cz0 - D0) - sz0; // parity-0 point of the next plane, from the tile's first
+  // what the thread stores: fine row h (of its two) in planes of parity p
+  // from zs; with d.xs2, the x tile lies two points further in every other
+  // row or plane (the tile 0 rows keep their first points)
+  bool vst[2][2];
+#pragma unroll
+  for (int h = 0; h < 2; ++h)
+#pragma unroll
+    for (int p = 0; p < 2; ++p) {
+      const int y = geo.f0[1] + ys0 + h - sy0;
+      const int sh = (int)((y * dsy + (geo.f0[2] + zs + p) * dsz) & d.xs2); // 0 or 2
+      const int x = fx0 + my_fx - geo.x0; // from the x tile's start
+      vst[h][p] = tact && my_fx < nfx && ys0 + h >= sy0 && ys0 + h < sy0 + nfy &&
+                  (d.xs2 == 0 || ((geo.x0 <= 0 || x >= sh) && x < d.xw + sh));
+    }
+  const double *const ycol = xrows + (my_cyr - LO) * XR + my_fx + (sx0 & 1);
   double w[8];
 #pragma unroll
   for (int k = 0; k < 8; ++k) w[k] = (NTL == 1 || (TK != T_ENO && k >= NTL)) ? 0.0 : d.w[k];
-
-  double yq[NTL][2][Q];
+  typename F::template Line<FMA, false> zl[NTL][2];
+  // store address of the parity-0 point of plane cz (base cz - D0), and from
+  // there to the parity-1 point that the same plane completes (base cz - D1)
+  double *oz = d.dst + (d.doff[0] + fx0 + my_fx) + (long long)(d.doff[1] + geo.f0[1] + ys0 - sy0) * dsy +
+               (long long)(d.doff[2] + geo.f0[2] + zs) * dsz;
+  constexpr int ODD = 1 - 2 * (D1 - D0);
+  const long long odd = ODD * dsz;
+  const double *col = nullptr; // of the next plane
+  auto plane = [&](auto U) {   // y and z passes of a plane, U its phase
+    const bool z0 = zs >= 0 && zs < nfz, z1 = zs + ODD >= 0 && zs + ODD < nfz;
 #pragma unroll
-  for (int t = 0; t < NTL; ++t)
+    for (int h = 0; h < 2; ++h) {
+      double e[NTL], o[NTL];
 #pragma unroll
-    for (int h = 0; h < 2; ++h)
-#pragma unroll
-      for (int q = 0; q < Q; ++q) yq[t][h][q] = 0.0;
-
-  // o0: this thread's store address in fine plane 2 * (cz0 + p - HI), carried
-  // by the multi-timelevel loop (the one-timelevel loop computes it here)
-  auto yzpass = [&](auto Ut, int p, const double *__restrict__ xr, double *o0) {
-    constexpr int U = decltype(Ut)::value;
-    if (!wact) return; // warp-uniform
-#pragma unroll
-    for (int t = 0; t < NTL; ++t) {
-      const double *col = xr + t * CY * XR + ycol;
-      auto get = [&](int m) { return col[m * XR]; };
-      yq[t][0][U] = F::template next<FMA>(0, get);
-      yq[t][1][U] = F::template next<FMA>(1, get);
+      for (int t = 0; t < NTL; ++t) {
+        const double *c = col + t * (rows * XR);
+        zl[t][h].template push<decltype(U)::value>(F::template next<FMA>(h, [&](int m) { return c[m * XR]; }), e[t],
+                                                   o[t]);
+      }
+      const double r0 = tcombine<FMA, TK, NTL>(w, e), r1 = tcombine<FMA, TK, NTL>(w, o);
+      double *const oh = h ? oz + dsy : oz;
+      if (z0 && vst[h][0]) *oh = r0;
+      if (z1 && vst[h][1]) oh[odd] = r1;
     }
-    const int cb = cz0 + p - HI;
-#pragma unroll
-    for (int zp = 0; zp < 2; ++zp) {
-      const int zs = 2 * cb + zp;
-      const bool zok = zs >= sz0 && zs < sz0 + nfz; // uniform
-      double *o;
-      if constexpr (SPLIT) o = obase + (long long)zs * dsz;
-      else o = zp ? o0 + dsz : o0;
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        double v[NTL];
-#pragma unroll
-        for (int t = 0; t < NTL; ++t)
-          v[t] = F::template next<FMA>(zp, [&](int m) { return yq[t][h][(U + 1 + (m - LO)) % Q]; });
-        const double r = tcombine<FMA, TK, NTL>(w, v);
-        if (zok && (h ? v1 : v0)) o[h ? dsy : 0] = r;
+    col += BY * XR;
+    oz += 2 * dsz;
+    zs += 2;
+  };
+  int phase = 0; // of the z lines' next push
+  for (int s = 0; s < nstages; ++s) {
+    const unsigned slot = (g0 + (unsigned)s) & 1u;
+    const int np = min(BZ, nplanes - s * BZ);
+    bool ok = true;
+    if constexpr (TMA) {
+      ok = mbar_wait_bounded(&ring.bars[slot], ((g0 + (unsigned)s) >> 1) & 1u);
+    } else {
+      cp_async_wait<1>();
+      __syncthreads();
+    }
+    if (ok && tid < (NTL == 1 ? np * BY : NTL * rows)) x_row<F, FMA>(xsrc + slot * (NTL * S::TLS), xdst, xs, nbx);
+    if constexpr (TMA) {
+      if (__syncthreads_or(!ok)) { // a wait gave up
+        // wait (bounded) for the next stage too, which is still in flight,
+        // so that no copy lands after the CTA has left
+        if (tid == 0) {
+          if (status) atomicCAS(status, 0, CGX_EDEVICE);
+          const unsigned g = g0 + (unsigned)s + 1u;
+          if (s + 1 < nstages) mbar_wait_bounded(&ring.bars[g & 1u], (g >> 1) & 1u);
+          if (!(ring.skip && g == 1u)) mbar_wait_bounded(&ring.bars[slot], ((g - 1u) >> 1) & 1u);
+        }
+        __syncthreads();
+        return false;
+      }
+      if (tid == 0 && s + 2 < nstages) issue(s + 2);
+    } else {
+      __syncthreads();
+      if (s + 2 < nstages) fetch(s + 2);
+      cp_async_commit();
+    }
+    if (wact) { // warp-uniform
+      col = ycol;
+      if constexpr (BZS > 0) { // whole turns of the phases
+        static_for<BZS>([&](auto P) {
+          if ((decltype(P)::value) < np) plane(std::integral_constant<int, decltype(P)::value % F::PHASES>());
+        });
+      } else {
+#pragma unroll 1
+        for (int p = 0; p < np; ++p) {
+          by_phase<F::PHASES>(phase, plane);
+          if (++phase == F::PHASES) phase = 0;
+        }
       }
     }
-  };
-
-  // Pipeline as in prolong_tile, one barrier per plane; the elected thread
-  // stages plane i + PD at the start of iteration i, into the slot last read
-  // by the x pass of plane i + PD - NB = i - 2.
-  if (tid == 0) {
-#pragma unroll
-    for (int p = 0; p < PD; ++p)
-      if (p < nplanes) issue(p);
+    if (TMA && s + 1 < nstages) __syncthreads(); // the x-pass rows are free
   }
-  // One-timelevel iteration i: stage plane i + PD; wait for plane i (the
-  // barrier also reduces the waits' failures, __syncthreads_or), run its x
-  // pass (DX: i < nplanes) and the y/z pass of plane i - 1 (DY: i >= 1).
-  // Multi-timelevel iteration i (iteration_rt): stage plane i + PD, run the
-  // y/z pass of plane i - 1 first -- on x-pass rows finished before the
-  // previous iteration's barrier -- which gives the copies of plane i a
-  // long pass's time to land, then wait for plane i, run its x pass, and
-  // end with the barrier.  With
-  // SPLIT (one timelevel: a short loop body) the whole groups of Q
-  // iterations run without per-iteration checks and a second unrolled copy
-  // handles the last ones.
-  bool ok = true;
-  auto iteration = [&](auto Ut, int i, auto DX, auto DY) {
-    constexpr bool X = decltype(DX)::value, Y = decltype(DY)::value;
-    if (!ok) return; // uniform: a wait gave up
-    if (tid == 0 && i + PD < nplanes) issue(i + PD);
-    const unsigned g = g0 + (unsigned)i;
-    const int fail = X ? !mbar_wait_bounded(&ring.bars[g % NB], (g / NB) & 1) : 0;
-    if (__syncthreads_or(fail)) {
-      if (tid == 0) *ring.abort = 1;
-      ok = false;
-      return;
-    }
-    if (X) xpass((int)(g % NB), xrows + (i & 1) * S::xbuf);
-    if (Y) yzpass(Ut, i - 1, xrows + ((i - 1) & 1) * S::xbuf, nullptr);
-  };
-  // the same iteration with run-time checks, one unrolled copy: the loop of
-  // the multi-timelevel variants, whose long bodies make a second unrolled
-  // copy (and its register allocation) cost more than the checks.  Its
-  // plane-dependent addresses are carried from one iteration to the next
-  // rather than recomputed: the ring slot and phase of plane i (slot
-  // (g0 + i) % NB, phase (g0 + i) / NB), the x-pass rows of planes i and
-  // i - 1, and the store address of the y/z pass's plane i - 1.
-  int rslot = (int)(g0 % NB);
-  unsigned rpar = (g0 / NB) & 1;
-  double *oz = obase + (long long)(2 * (cz0 - HI)) * dsz;
-  const long long dz2 = 2 * dsz;
-  double *xcur = xrows, *xprev = xrows + S::xbuf; // x-pass rows of planes i, i - 1
-  auto iteration_rt = [&](auto Ut, int i) {
-    if (tid == 0 && i + PD < nplanes) issue(i + PD);
-    if (i >= 1) {
-      yzpass(Ut, i - 1, xprev, oz);
-      oz += dz2;
-    }
-    const bool landed = i < nplanes && mbar_wait_bounded(&ring.bars[rslot], rpar);
-    if (landed) xpass(rslot, xcur);
-    double *const xt = xcur;
-    xcur = xprev;
-    xprev = xt;
-    if (++rslot == NB) {
-      rslot = 0;
-      rpar ^= 1u;
-    }
-    if (__syncthreads_or(i < nplanes && !landed)) { // a wait gave up
-      if (tid == 0) *ring.abort = 1;
-      ok = false;
-    }
-  };
-  using T_ = std::true_type;
-  using F_ = std::false_type;
-  int i0 = 1;
-  if (SPLIT) {
-    iteration(std::integral_constant<int, Q - 1>(), 0, T_(), F_());
-    // whole groups of Q iterations with both passes, then the last ones
-    for (; ok && i0 + Q <= nplanes; i0 += Q)
-      static_for<Q>([&](auto Ut) { iteration(Ut, i0 + decltype(Ut)::value, T_(), T_()); });
-    static_for<Q>([&](auto Ut) {
-      const int i = i0 + decltype(Ut)::value;
-      if (ok && i < nplanes) iteration(Ut, i, T_(), T_());
-      else if (ok && i == nplanes) iteration(Ut, i, F_(), T_());
-    });
-  } else {
-    iteration_rt(std::integral_constant<int, Q - 1>(), 0);
-    for (; ok && i0 <= nplanes; i0 += Q)
-      static_for<Q>([&](auto Ut) {
-        const int i = i0 + decltype(Ut)::value;
-        if (ok && i <= nplanes) iteration_rt(Ut, i);
-      });
-  }
-  if (!ok) {
-    // a wait gave up: wait (bounded) for every plane staged, so that no
-    // copy lands after the CTA has left
-    if (tid == 0) {
-      if (status) atomicCAS(status, 0, CGX_EDEVICE);
-      for (int i = 0; i < issued; ++i) {
-        if (i == skip) continue;
-        const unsigned g = g0 + (unsigned)i;
-        mbar_wait_bounded(&ring.bars[g % NB], (g / NB) & 1);
-      }
-    }
-    __syncthreads();
-    return false;
-  }
-  ring.g = g0 + (unsigned)nplanes;
+  ring.g = g0 + (unsigned)nstages;
+  if constexpr (!TMA) cp_async_wait<0>();
   __syncthreads(); // shared memory free for the next tile
   return true;
 }
