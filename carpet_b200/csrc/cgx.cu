@@ -134,12 +134,13 @@ int ceil_div(int a, int b) { return (a + b - 1) / b; }
 // against 520 us), and for more timelevels, which are bound by their
 // arithmetic, only where they cost none (the boundary slabs of 129^3 levels:
 // 176 us with sector tiles, a tenth more tiles, against 168 us).
-long long prolong_tiles(Desc &d, int config, int pzmax) {
+// prolong_xy lays out x and y (false: no tile fits), prolong_z then z.
+bool prolong_xy(Desc &d, int config) {
   const TmaCfg &c = TMA_CFGS[config];
   const int W = stencil_width(d), ntl = std::min(3, std::max(1, (int)d.ntl));
   const int fixed = tma_planes(family_phases(d.kind, d.order), ntl); // planes per stage, or 0
   const int rpt = tma_rpt(W, c.nt, c.pyc, ntl, fixed), tls = tma_tls(W, c.nt, c.pyc, ntl, fixed);
-  const int yo = d.soff[1] & 1, zo = d.soff[2] & 1;
+  const int yo = d.soff[1] & 1;
   const int nu = ceil_div(d.n[0], PTXMAX), po = d.soff[0] & 1;
   struct XTiles {
     int ptx, xw, xo, xs2, nbx, bx, nx, ptyc, ny;
@@ -171,29 +172,37 @@ long long prolong_tiles(Desc &d, int config, int pzmax) {
     else if (d.dsy % 2 == 0 && d.dsz % 2 == 0) s = rows({PTXMAX, 12, xo, 2, (d.soff[0] - xo) % 2 == 0 ? 7 : 8});
     if (s.ny && (x.ny == 0 || (long long)s.nx * s.ny * 2 <= (long long)x.nx * x.ny * (ntl == 1 ? 3 : 2))) x = s;
   }
-  if (x.ny == 0) return -1;
-  const int by = x.ptyc + W;
-  const int ntz = ceil_div(d.n[2] + zo, pzmax);
-  const int pz = (ceil_div(d.n[2] + zo, ntz) + 1) & ~1;
-  const int planes = pz / 2 + W, pmax = std::min(rpt / by, tls / (x.bx * by));
-  const int stages = ceil_div(planes, fixed ? fixed : pmax);
+  if (x.ny == 0) return false;
   d.ptx = (unsigned char)x.ptx;
   d.xw = (unsigned char)x.xw;
   d.xo = (unsigned char)x.xo;
   d.xs2 = (unsigned char)x.xs2;
   d.ptyc = (unsigned char)x.ptyc;
   d.bx = (unsigned char)x.bx;
-  d.by = (unsigned char)by;
-  d.bz = (unsigned char)(fixed ? fixed : ceil_div(planes, stages));
-  d.pz = (short)pz;
+  d.by = (unsigned char)(x.ptyc + W);
   d.rpx = ceil_div(65536, x.ptx);
   d.tma = 0;
   d.tiles[0] = x.nx;
   d.tiles[1] = x.ny;
-  d.tiles[2] = ceil_div(d.n[2] + zo, pz);
   division_magic(d.tiles[0], &d.mg[0], &d.sh[0]);
   division_magic(d.tiles[1], &d.mg[1], &d.sh[1]);
+  return true;
+}
+long long prolong_z(Desc &d, int config, int pzmax) {
+  const TmaCfg &c = TMA_CFGS[config];
+  const int W = stencil_width(d), ntl = std::min(3, std::max(1, (int)d.ntl)), zo = d.soff[2] & 1;
+  const int fixed = tma_planes(family_phases(d.kind, d.order), ntl);
+  const int rpt = tma_rpt(W, c.nt, c.pyc, ntl, fixed), tls = tma_tls(W, c.nt, c.pyc, ntl, fixed);
+  const int ntz = ceil_div(d.n[2] + zo, pzmax);
+  const int pz = (ceil_div(d.n[2] + zo, ntz) + 1) & ~1, planes = pz / 2 + W;
+  const int stages = ceil_div(planes, fixed ? fixed : std::min(rpt / d.by, tls / (d.bx * d.by)));
+  d.bz = (unsigned char)(fixed ? fixed : ceil_div(planes, stages));
+  d.pz = (short)pz;
+  d.tiles[2] = ceil_div(d.n[2] + zo, pz);
   return (long long)d.tiles[0] * d.tiles[1] * d.tiles[2];
+}
+long long prolong_tiles(Desc &d, int config, int pzmax) {
+  return prolong_xy(d, config) ? prolong_z(d, config, pzmax) : -1;
 }
 
 // The most fine z points per tile for prolongation descriptors that run in
@@ -202,47 +211,119 @@ long long prolong_tiles(Desc &d, int config, int pzmax) {
 // planes' time of set-up and first copies; a launch takes its total over the
 // slots, and one tile at the least.  Many tiles take the configuration's pz
 // (halo planes cost), few are cut in z until the slots are filled: one
-// 64 x 12 x 52 region is 4 tiles of 31 planes uncut and took 78 us.
+// 64 x 12 x 52 region is 4 tiles of 31 planes uncut and took 78 us, 17 us cut.
 constexpr int SM_COUNT = 148;
-int choose_pz(const std::vector<const Desc *> &ds, int config) {
-  int best = TMA_CFGS[config].pz;
-  double best_cost = -1.0;
-  for (int pz = best; pz >= 4; pz /= 2) {
-    double sum = 0.0, longest = 0.0;
-    for (const Desc *p : ds) {
-      Desc d = *p;
-      const long long nt = prolong_tiles(d, config, pz);
-      if (nt <= 0) continue;
-      const double cost = d.pz / 2 + stencil_width(d) + 4;
-      sum += nt * cost;
-      longest = std::max(longest, cost);
-    }
-    const double t = sum / (SM_COUNT * TMA_CFGS[config].mb) + longest;
-    if (best_cost < 0.0 || t < best_cost) {
-      best_cost = t;
-      best = pz;
+struct PzCost { // of the candidates pz, pz / 2, ... 4 of a configuration
+  static constexpr int NC = 5;
+  int pz0, slots;
+  double sum[NC] = {}, longest[NC] = {};
+  explicit PzCost(int config) : pz0(TMA_CFGS[config].pz), slots(SM_COUNT * TMA_CFGS[config].mb) {}
+  void add(const Desc &d) { // tiled in x and y
+    const int zo = d.soff[2] & 1, W = stencil_width(d), n = d.n[2] + zo;
+    for (int c = 0; c < NC && pz0 >> c >= 4; ++c) {
+      const int pz = (ceil_div(n, ceil_div(n, pz0 >> c)) + 1) & ~1;
+      const double cost = pz / 2 + W + 4;
+      sum[c] += (double)d.tiles[0] * d.tiles[1] * ceil_div(n, pz) * cost;
+      longest[c] = std::max(longest[c], cost);
     }
   }
-  return best;
+  int best() const {
+    int b = 0;
+    for (int c = 1; c < NC && pz0 >> c >= 4; ++c)
+      if (sum[c] / slots + longest[c] < sum[b] / slots + longest[b]) b = c;
+    return pz0 >> b;
+  }
+};
+long long prolong_tiles_alone(Desc &d, int config) { // one descriptor launched alone
+  if (!prolong_xy(d, config)) return -1;
+  PzCost c(config);
+  c.add(d);
+  return prolong_z(d, config, c.best());
 }
 
-// Tiles of a descriptor launched alone.  Prolongation: the cp.async kernels'
-// configuration.  Copy and restriction: STILE consecutive points of the
-// flattened region.
+// Units per row of a copy (Sector, cgx_device.cuh): those of the most sectors
+// that a row of the region touches, whatever its alignment, in pairs; 0 for
+// rows that go point by point.
+int row_units(const Desc &d) {
+  if (d.kind != K_COPY || d.n[0] < SECTOR_ROW) return 0;
+  int most = 3; // points before the region in a row's first sector
+  if (d.dst && d.dsy % 4 == 0 && d.dsz % 4 == 0)
+    most = (int)((reinterpret_cast<uintptr_t>(d.dst) / 8 + d.doff[0] + d.doff[1] * d.dsy + d.doff[2] * d.dsz) & 3);
+  const int ns = 2 * ceil_div(d.n[0] + most, 8);
+  return 4LL * ns * d.n[1] * d.n[2] < (1LL << 31) ? ns : 0;
+}
+
+// cuTensorMapEncodeTiled from the driver, found once; null without a driver
+PFN_cuTensorMapEncodeTiled_v12000 tma_encoder() {
+  static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
+  static bool tried = false;
+  if (!tried) {
+    tried = true;
+    void *p = nullptr;
+    cudaDriverEntryPointQueryResult q = cudaDriverEntryPointSymbolNotFound;
+    if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &q) ==
+            cudaSuccess &&
+        q == cudaDriverEntryPointSuccess)
+      fn = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(p);
+    else
+      cudaGetLastError();
+  }
+  return fn;
+}
+
+// The tensor-copy unit can address the source arrays of a prolongation that
+// has a TMA variant: 16-byte aligned bases, row and plane pitches that are
+// multiples of 16 bytes.
+bool tma_addressable(const Desc &d) {
+  if (!is_stencil(d.kind) || tma_variant(d) < 0 || !tma_encoder()) return false;
+  if (d.ssy % 2 || d.ssz % 2 || d.ssz >= (1LL << 37)) return false;
+  for (int t = 0; t < d.ntl; ++t)
+    if (reinterpret_cast<uintptr_t>(d.src[t]) % 16) return false;
+  return true;
+}
+
+// Tiles of a streaming kind: STILE or HTILE units of the flattened region
+// (cgx_device.cuh).  ns: a copy's units per row, or 0.
+long long stream_tiles(Desc &d, int ns) {
+  if ((long long)d.n[0] * d.n[1] * d.n[2] >= (1LL << 31)) return -1;
+  long long row = d.n[0], planes = d.n[2];
+  int per = STILE;
+  d.ns = ns;
+  if (ns) {
+    row = ns;
+    per = STILE / 4;
+  } else if (d.kind == K_PROLONG_MONO) {
+    row = d.ns = ((d.soff[0] + d.n[0] - 1) >> 1) - (d.soff[0] >> 1) + 1;
+    per = HTILE;
+  } else if (d.kind == K_RESTRICT_CC || d.kind == K_RESTRICT_CC3) {
+    per = HTILE;
+  } else if (d.kind == K_RESTRICT_CC5) {
+    planes = (planes + 1) / 2;
+    per = HTILE;
+  }
+  d.tiles[0] = (int)((row * d.n[1] * planes + per - 1) / per);
+  d.tiles[1] = d.tiles[2] = 1;
+  division_magic((int)row, &d.mg[0], &d.sh[0]);
+  division_magic(d.n[1], &d.mg[1], &d.sh[1]);
+  return d.tiles[0];
+}
+
+// Tiles of a descriptor launched alone.  Prolongation: staged by TMA where the
+// arrays allow it (d.tma), else by cp.async.
 int kind_tiles(Desc &d) {
   const int kind = d.kind;
   const bool prol = is_stencil(kind);
   long long tot = 1;
   if (prol) {
-    tot = prolong_tiles(d, PLAIN_CFG, choose_pz({&d}, PLAIN_CFG));
+    // a box's tensor maps cost the call about 1 us per timelevel: staged by
+    // TMA from 2^18 source values on (161^3, order 5: 37 -> 16 us a call; a
+    // slab of 64 x 12 x 52 with three timelevels 18.0 against 17.3 us)
+    const bool big = (long long)d.n[0] * d.n[1] * d.n[2] * d.ntl >= 8LL << 18;
+    const int cfg = big && tma_addressable(d) ? BOX_CFG : PLAIN_CFG;
+    tot = prolong_tiles_alone(d, cfg);
+    d.tma = tot > 0 && cfg == BOX_CFG;
   } else {
-    const long long npts = (long long)d.n[0] * d.n[1] * d.n[2];
-    if (npts >= (1LL << 31)) return -1;
-    d.tiles[0] = (int)((npts + STILE - 1) / STILE);
-    d.tiles[1] = d.tiles[2] = 1;
-    tot = d.tiles[0];
-    division_magic(d.n[0], &d.mg[0], &d.sh[0]);
-    division_magic(d.n[1], &d.mg[1], &d.sh[1]);
+    tot = stream_tiles(d, row_units(d));
   }
   return tot > 0x7fffffff ? -1 : (int)tot;
 }
@@ -781,9 +862,22 @@ int launch_staged(Built &b, int fp, int *status, cudaStream_t s) {
   return rc;
 }
 
+// A box tiled for TMA.  Its tensor maps are encoded here, on each launch.
+int launch_box(const Desc &d, int ntiles, int fp, int *status, cudaStream_t s) {
+  CUtensorMap maps[3] = {};
+  Desc t = d;
+  if (!encode_tma_maps(t, maps)) return fail(CGX_ECUDA, "transfer: a tensor map could not be encoded");
+  const int v = tma_variant(d);
+  const bool f = fp == CGX_FP_FMA;
+  if (v >= TV_TUNED) return klaunch_box_eno(f, v, d, maps, ntiles, status, s);
+  if (v / 4 >= 5) return f ? klaunch_box_f1_p1(v, d, maps, ntiles, status, s) : klaunch_box_f0_p1(v, d, maps, ntiles, status, s);
+  return f ? klaunch_box_f1_p0(v, d, maps, ntiles, status, s) : klaunch_box_f0_p0(v, d, maps, ntiles, status, s);
+}
+
 int launch_pair(const Desc &d, int ntiles, int fp, int *status, cudaStream_t s) {
   const bool high = d.kind == K_PROLONG_VC && d.order >= 7;
   if (high) return klaunch_pair_hi(fp, d, ntiles, status, s);
+  if (is_stencil(d.kind) && d.tma) return launch_box(d, ntiles, fp, status, s);
   if (!is_stencil(d.kind))
     return fp == CGX_FP_FMA ? klaunch_spair_f1(d, ntiles, status, s) : klaunch_spair_f0(d, ntiles, status, s);
   return fp == CGX_FP_FMA ? klaunch_pair_f1(d, ntiles, status, s) : klaunch_pair_f0(d, ntiles, status, s);
@@ -831,7 +925,9 @@ int launch_map_capped(int fp, const Desc *d, const CUtensorMap *maps, const int2
     if (i < TV_COUNT) {
       const int k = cfg ? cfg[i] : 0;
       if (k < 0 || k >= TMA_NCFG) return fail(CGX_EINVAL, "bad tile configuration %d", k);
-      rc = kTmaLaunch[f][i / 4 >= 5][tma_kernel_cfg(k)](i | (g_debug_skip_tma ? 1 << 30 : 0), d, maps, tm, n, c, status, s);
+      const int v = i | (g_debug_skip_tma ? 1 << 30 : 0);
+      rc = i >= TV_TUNED ? klaunch_tma_eno(f, v, d, maps, tm, n, c, status, s)
+                         : kTmaLaunch[f][i / 4 >= 5][tma_kernel_cfg(k)](v, d, maps, tm, n, c, status, s);
     } else if (i == SEG_STENCIL) {
       rc = f ? klaunch_map_f1(d, tm, n, c, status, s) : klaunch_map_f0(d, tm, n, c, status, s);
     } else {
@@ -841,35 +937,6 @@ int launch_map_capped(int fp, const Desc *d, const CUtensorMap *maps, const int2
     if (rc) return rc;
   }
   return CGX_OK;
-}
-
-// cuTensorMapEncodeTiled from the driver, found once; null without a driver
-PFN_cuTensorMapEncodeTiled_v12000 tma_encoder() {
-  static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
-  static bool tried = false;
-  if (!tried) {
-    tried = true;
-    void *p = nullptr;
-    cudaDriverEntryPointQueryResult q = cudaDriverEntryPointSymbolNotFound;
-    if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &q) ==
-            cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      fn = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(p);
-    else
-      cudaGetLastError();
-  }
-  return fn;
-}
-
-// The tensor-copy unit can address the source arrays of a prolongation that
-// has a TMA variant: 16-byte aligned bases, row and plane pitches that are
-// multiples of 16 bytes.
-bool tma_addressable(const Desc &d) {
-  if (!is_stencil(d.kind) || tma_variant(d) < 0 || !tma_encoder()) return false;
-  if (d.ssy % 2 || d.ssz % 2 || d.ssz >= (1LL << 37)) return false;
-  for (int t = 0; t < d.ntl; ++t)
-    if (reinterpret_cast<uintptr_t>(d.src[t]) % 16) return false;
-  return true;
 }
 
 } // namespace
@@ -1147,13 +1214,27 @@ int cgx_batch_upload(cgx_batch *b, void *stream) {
   std::map<int, std::vector<int>> by_variant;
   for (int i : order)
     if (is_stencil(dq[i].kind)) by_variant[tma_addressable(dq[i]) ? tma_variant(dq[i]) : -1].push_back(i);
+  // Copies go by sectors where hardly any of the batch's copied points lie in
+  // narrow rows: a ghost sync, a third of whose points do, stays one kernel
+  // (with two, its halves would be forked and joined at every phase).
+  long long narrow = 0, copied = 0;
+  for (int i : order)
+    if (dq[i].kind == K_COPY) {
+      copied += b->points[i];
+      narrow += dq[i].ns ? 0 : b->points[i];
+    }
+  if (8 * narrow > copied)
+    for (int i : order)
+      if (dq[i].kind == K_COPY && dq[i].ns) ntq[i] = stream_tiles(dq[i], 0);
   for (const auto &kv : by_variant) {
-    const int cfg = kv.first >= 0 ? b->tma_cfg[kv.first] : PLAIN_CFG;
-    std::vector<const Desc *> ds;
-    for (int i : kv.second) ds.push_back(&dq[i]);
-    const int pz = choose_pz(ds, cfg);
+    const int cfg = kv.first >= 0 ? tma_cfg(kv.first, b->tma_cfg[kv.first]) : PLAIN_CFG;
+    PzCost cost(cfg);
+    for (int i : kv.second)
+      if (prolong_xy(dq[i], cfg)) cost.add(dq[i]);
+      else return fail(CGX_EINVAL, "batch: region too large");
+    const int pz = cost.best();
     for (int i : kv.second) {
-      const long long nt = prolong_tiles(dq[i], cfg, pz);
+      const long long nt = prolong_z(dq[i], cfg, pz);
       if (nt <= 0 || nt >= (1LL << 31)) return fail(CGX_EINVAL, "batch: region too large");
       ntq[i] = nt;
       if (kv.first >= 0 && !encode_tma_maps(dq[i], &em[3 * (size_t)i]))
@@ -1297,14 +1378,14 @@ int cgx_batch_launch(cgx_batch *b, void *stream) {
 // the fastest; then upload with the choices.  Repeated launches of a batch write the same values
 // (pairs write disjoint points and read none of them), so tuning on the
 // caller's own data is safe.
-static_assert(CGX_TMA_VARIANTS == TV_COUNT && CGX_TMA_CONFIGS == TMA_NCFG, "tuning constants of the C-ABI");
+static_assert(CGX_TMA_VARIANTS == TV_TUNED && CGX_TMA_CONFIGS == TMA_NCFG, "tuning constants of the C-ABI");
 int cgx_batch_autotune(cgx_batch *b, int reps, void *stream, int *chosen) {
   if (!b || reps < 1) return fail(CGX_EINVAL, "autotune: bad arguments");
   cudaStream_t s = (cudaStream_t)stream;
   int rc = cgx_batch_upload(b, stream);
   if (rc) return rc;
-  bool present[TV_COUNT];
-  for (int v = 0; v < TV_COUNT; ++v) present[v] = b->seg[v + 1] > b->seg[v];
+  bool present[TV_TUNED];
+  for (int v = 0; v < TV_TUNED; ++v) present[v] = b->seg[v + 1] > b->seg[v];
   // each launch timed on its own; a configuration scores the median
   std::vector<cudaEvent_t> ev(2 * (size_t)reps, nullptr);
   cudaError_t e = cudaSuccess;
@@ -1323,7 +1404,7 @@ int cgx_batch_autotune(cgx_batch *b, int reps, void *stream, int *chosen) {
     return launch_map(b->fp_mode, b->d_descs, b->d_maps, b->d_tmap, sg, b->tma_cfg, b->d_counter,
                       b->d_status, s);
   };
-  for (int v = 0; v < TV_COUNT && rc == CGX_OK; ++v) {
+  for (int v = 0; v < TV_TUNED && rc == CGX_OK; ++v) {
     if (!present[v]) continue;
     int best = 0;
     float best_ms = 0.f;
@@ -1353,12 +1434,12 @@ int cgx_batch_autotune(cgx_batch *b, int reps, void *stream, int *chosen) {
   for (auto x : ev) cudaEventDestroy(x);
   if (rc) return rc;
   if (chosen)
-    for (int v = 0; v < TV_COUNT; ++v) chosen[v] = present[v] ? b->tma_cfg[v] : -1;
+    for (int v = 0; v < TV_TUNED; ++v) chosen[v] = present[v] ? b->tma_cfg[v] : -1;
   return cgx_batch_upload(b, stream);
 }
 
 int cgx_batch_set_config(cgx_batch *b, int variant, int config) {
-  if (!b || variant < -1 || variant >= TV_COUNT || config < 0 || config >= TMA_NCFG)
+  if (!b || variant < -1 || variant >= TV_TUNED || config < 0 || config >= TMA_NCFG)
     return fail(CGX_EINVAL, "set_config: variant %d / configuration %d out of range", variant, config);
   for (int v = 0; v < TV_COUNT; ++v)
     if (variant < 0 || v == variant) b->tma_cfg[v] = config;
@@ -1572,7 +1653,7 @@ int cgx_chain_upload(cgx_chain *c, void *stream) {
                         "(16-byte aligned base, even row and plane pitch)",
                         j, i);
         } else if ((d.kind == K_COPY && d.ntl == 1) || d.kind == K_RESTRICT_VC) {
-          nt = b->ntiles[i];
+          nt = stream_tiles(d, 0);
         } else {
           return fail(CGX_EUNSUPPORTED,
                       "chain: batch %zu pair %d: only vertex-centred prolongation, one-timelevel "
@@ -1763,9 +1844,11 @@ extern "C" int cgx_transfer_pairs_noalloc(const cgx_pair *pairs, int npairs, voi
                     i0 + i, b.d.order);
       hd[i] = b.d;
       hp[i] = tiles;
-      // a list of many pairs fills the GPU with whole-length tiles
-      if (npairs > SM_COUNT / 8 && is_stencil(b.d.kind))
-        b.ntiles = (int)prolong_tiles(hd[i], PLAIN_CFG, TMA_CFGS[PLAIN_CFG].pz);
+      // the cp.async kernels' tiles; a list of many pairs fills the GPU with
+      // whole-length ones
+      if (is_stencil(b.d.kind))
+        b.ntiles = (int)(npairs > SM_COUNT / 8 ? prolong_tiles(hd[i], PLAIN_CFG, TMA_CFGS[PLAIN_CFG].pz)
+                                               : prolong_tiles_alone(hd[i], PLAIN_CFG));
       tiles += b.ntiles;
     }
     cudaError_t e = cudaMemcpyAsync(d_descs + i0, hd, n * sizeof(Desc), cudaMemcpyHostToDevice, s);
@@ -1899,7 +1982,8 @@ int launch_tile_map(const Desc *d_descs, const CUtensorMap *d_maps, const int2 *
 // A prolongation descriptor's tiles in TMA tile configuration `config`
 // (the tiling of a batch upload); returns the tile count, <= 0 if none.
 long long tile_prolongation(Desc &d, int config) {
-  return prolong_tiles(d, config, TMA_CFGS[config].pz);
+  const int c = config < 0 ? PLAIN_CFG : tma_cfg(tma_variant(d), config);
+  return prolong_tiles(d, c, TMA_CFGS[c].pz);
 }
 
 bool encode_tma_maps(Desc &d, CUtensorMap maps[3]) {

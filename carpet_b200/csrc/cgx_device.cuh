@@ -61,10 +61,10 @@ struct Desc {
   unsigned char xs2;
   unsigned char pad0;
   int rpx; // ceil(65536 / ptx): t / ptx = t * rpx >> 16 for t < 256
-  int pad1;
+  int ns;  // copies: units per row (Sector), 0: point by point; monotone prolongation: coarse bases per row
   long long ssy, ssz; // source strides (elements) in y and z
   long long dsy, dsz; // destination strides
-  unsigned mg[2]; // division magic (div_magic) for n[0], n[1]; prolongation: tiles[0], tiles[1]
+  unsigned mg[2]; // division magic (div_magic) for ns or n[0], n[1]; prolongation: tiles[0], tiles[1]
   int sh[2];
   const double *src[3];
   double *dst;
@@ -415,9 +415,26 @@ template <int N> __device__ __forceinline__ void cp_async_wait() {
 // zones are 3 points thin in one direction.  A tile is STILE consecutive
 // points of the region flattened x-fastest, run by the LANES threads of a
 // CTA: every lane is busy whatever the shape, consecutive lanes touch
-// consecutive x, and each thread issues a group of loads before its stores.  A flat index is split into (i, j, k) by
-// 32-bit multiply-high with precomputed magic numbers.
+// consecutive x, and each thread issues a group of loads before its stores.
+// A flat index is split into (i, j, k) by 32-bit multiply-high with
+// precomputed magic numbers.
+//
+// Copies whose rows have SECTOR_ROW points or more go by destination sectors
+// (32 bytes; d.ns): two threads take two neighbouring sectors, each thread
+// one half of either, so that a warp's two 16-byte stores cover whole sectors
+// -- L2 fetches the rest of a sector that a store covers in part from DRAM --
+// and an index is split once for four points: of 60 instructions per point
+// the point-by-point form spent most on that, and half of the issue slots.  A
+// tile is then STILE / 4 threads' worth.  They are kernels of their own: in
+// one kernel with the point form, inlined or as calls, the latter lost its
+// eight loads in flight (211 -> 260 to 373 us).
 constexpr int STILE = 1024;
+constexpr int SECTOR_ROW = 16; // narrower rows have hardly a whole sector
+// The kinds that compute much per point (8 to 216 source values) take tiles
+// of HTILE units, one or two per thread: their regions are small (a coarse
+// patch of 20^3 points is 8 tiles of 1024) and eight points of a thread ran
+// one after another on a GPU two thirds idle.
+constexpr int HTILE = 256;
 
 // The streaming kinds, one persistent kernel each.
 enum StreamVariant : int {
@@ -430,8 +447,9 @@ enum StreamVariant : int {
   SV_RESTRICT_CC3 = 6, // third-order cell-centred restriction
   SV_RESTRICT_CC5 = 7, // fifth-order cell-centred restriction
   SV_MONO = 8,         // monotone order-5 prolongation
-  SV_TIME = 9,         // time combination of temporaries (K_TIME)
-  SV_COUNT = 10
+  SV_SECTOR = 9,       // the four copies by destination sectors (d.ns), in the order above
+  SV_TIME = 13,        // time combination of temporaries (K_TIME)
+  SV_COUNT = 14
 };
 // A batch launches its segments in order: the time combination of staged
 // transfers must come after every kind that writes their temporaries.
@@ -445,9 +463,7 @@ template <class D> __host__ __device__ __forceinline__ int stream_variant(const 
   if (d.kind == K_TIME) return SV_TIME;
   if (d.kind == K_PROLONG_MONO) return SV_MONO;
   if (d.kind != K_COPY) return -1;
-  if (d.ntl == 1) return SV_COPY1;
-  if (d.ntl == 2) return SV_COPY2;
-  return d.tkind == T_ENO ? SV_COPY3E : SV_COPY3Q;
+  return (d.ns ? SV_SECTOR : SV_COPY1) + (d.ntl == 1 ? 0 : d.ntl == 2 ? 1 : d.tkind == T_ENO ? 3 : 2);
 }
 
 // Source loads of the streaming tiles: through the read-only path (__ldg)
@@ -479,6 +495,91 @@ __device__ __forceinline__ void unflatten(const D &d, unsigned p, int &i, int &j
 // group sizes: points whose loads a thread issues before it stores them
 template <int LANES, int NTL> __host__ __device__ constexpr int stream_group() {
   return (STILE / LANES) < (NTL == 1 ? 8 : 4) ? (STILE / LANES) : (NTL == 1 ? 8 : 4);
+}
+
+// Unit p of the region's destination rows, the rows' first and last sectors
+// whole: its row, and the x (-7 .. n[0] + 6) of its first half sector, which
+// starts on 16 bytes; the other half lies four points further.
+struct Sector {
+  int x, j, k;
+};
+template <class D> __device__ __forceinline__ Sector sector(const D &d, unsigned p, const double *dst) {
+  const unsigned q = div_magic(p, d.mg[0], d.sh[0]), r = div_magic(q, d.mg[1], d.sh[1]);
+  Sector s;
+  s.j = (int)(q - r * (unsigned)d.n[1]);
+  s.k = (int)r;
+  const unsigned at = (unsigned)(reinterpret_cast<uintptr_t>(dst) >> 3) + (unsigned)s.j * (unsigned)d.dsy +
+                      (unsigned)s.k * (unsigned)d.dsz;
+  const int u = (int)(p - q * (unsigned)d.ns);
+  s.x = 8 * (u >> 1) + 2 * (u & 1) - (int)(at & 3u);
+  return s;
+}
+// stores the points of a half sector that lie in the region; o: its first one
+__device__ __forceinline__ void store_half(double *o, int x, int n, double a, double b) {
+  if (x >= 0 && x + 1 < n) {
+    *reinterpret_cast<double2 *>(o) = make_double2(a, b);
+  } else {
+    if (x >= 0 && x < n) o[0] = a;
+    if (x + 1 >= 0 && x + 1 < n) o[1] = b;
+  }
+}
+// the source points of a half sector from s + x, those outside the row
+// replaced by its end points; one load where they start on 16 bytes too
+__device__ __forceinline__ void load_half(const double *s, int x, int n, double &a, double &b) {
+  if (x >= 0 && x + 1 < n && (reinterpret_cast<uintptr_t>(s + x) & 15) == 0) {
+    const double2 v = __ldg(reinterpret_cast<const double2 *>(s + x));
+    a = v.x;
+    b = v.y;
+  } else {
+    a = __ldg(s + min(max(x, 0), n - 1));
+    b = __ldg(s + min(max(x + 1, 0), n - 1));
+  }
+}
+
+template <int FMA, int NTL, int TK, int LANES, class D>
+__device__ __forceinline__ void copy_sectors(const D &d, int tile, int lid) {
+  constexpr int PER = STILE / 4 / LANES, G = NTL == 1 ? PER : 1; // units whose loads are issued before their stores
+  const unsigned nunits = (unsigned)d.ns * d.n[1] * d.n[2], p0 = (unsigned)tile * (STILE / 4) + lid;
+  const long long so = d.soff[0] + d.soff[1] * d.ssy + d.soff[2] * d.ssz;
+  double *dst = d.dst + (d.doff[0] + d.doff[1] * d.dsy + d.doff[2] * d.dsz);
+  double w[NTL == 1 ? 1 : 8];
+#pragma unroll
+  for (int k = 0; k < (NTL == 1 ? 1 : 8); ++k) w[k] = NTL == 1 ? 0.0 : d.w[k];
+#pragma unroll 1
+  for (int r0 = 0; r0 < PER; r0 += G) {
+    double v[G][NTL][4];
+    Sector c[G];
+#pragma unroll
+    for (int r = 0; r < G; ++r) {
+      const unsigned p = p0 + (r0 + r) * LANES;
+      if (p < nunits) {
+        c[r] = sector(d, p, dst);
+        const long long row = so + c[r].j * d.ssy + c[r].k * d.ssz;
+#pragma unroll
+        for (int t = 0; t < NTL; ++t)
+#pragma unroll
+          for (int h = 0; h < 2; ++h)
+            load_half(d.src[t] + row, c[r].x + 4 * h, d.n[0], v[r][t][2 * h], v[r][t][2 * h + 1]);
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < G; ++r) {
+      const unsigned p = p0 + (r0 + r) * LANES;
+      if (p < nunits) {
+        double o[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          double u[NTL];
+#pragma unroll
+          for (int t = 0; t < NTL; ++t) u[t] = v[r][t][e];
+          o[e] = tcombine<FMA, TK, NTL>(w, u);
+        }
+        double *out = dst + (c[r].x + c[r].j * d.dsy + c[r].k * d.dsz);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) store_half(out + 4 * h, c[r].x + 4 * h, d.n[0], o[2 * h], o[2 * h + 1]);
+      }
+    }
+  }
 }
 
 template <int FMA, int NTL, int TK, int LANES, class D, bool CG = false, int PTS = STILE, int GMAX = 8>
@@ -556,13 +657,15 @@ __device__ __forceinline__ void restrict_vc_tile(const D &d, int tile, int lid) 
 
 template <int FMA, int LANES, class D>
 __device__ __forceinline__ void restrict_cc_tile(const D &d, int tile, int lid) {
-  constexpr int PER = STILE / LANES;
+  constexpr int PER = HTILE / LANES;
   const unsigned npts = (unsigned)d.n[0] * d.n[1] * d.n[2];
-  const unsigned p0 = (unsigned)tile * STILE + lid;
+  const unsigned p0 = (unsigned)tile * HTILE + lid;
   const double *s0 = d.src[0] + (d.soff[0] + d.soff[1] * d.ssy + d.soff[2] * d.ssz);
   double *dst = d.dst + (d.doff[0] + d.doff[1] * d.dsy + d.doff[2] * d.dsz);
   const long long ssy = d.ssy, ssz = d.ssz;
   const double w = 0.125; // f1*f1*f1 with f1 = f2 = 1/2
+  // the two x neighbours in one load where every row starts on 16 bytes
+  const bool pairs = ((reinterpret_cast<uintptr_t>(s0) | (uintptr_t)(8 * ssy) | (uintptr_t)(8 * ssz)) & 15) == 0;
 #pragma unroll 2
   for (int r = 0; r < PER; ++r) {
     const unsigned p = p0 + r * LANES;
@@ -570,9 +673,11 @@ __device__ __forceinline__ void restrict_cc_tile(const D &d, int tile, int lid) 
     int i, j, k;
     unflatten(d, p, i, j, k);
     const double *q = s0 + 2 * (i + j * ssy + k * ssz);
-    const double a0 = __ldg(q), a1 = __ldg(q + 1), a2 = __ldg(q + ssy), a3 = __ldg(q + 1 + ssy);
-    const double a4 = __ldg(q + ssz), a5 = __ldg(q + 1 + ssz);
-    const double a6 = __ldg(q + ssy + ssz), a7 = __ldg(q + 1 + ssy + ssz);
+    auto pair = [&](const double *u) {
+      return pairs ? __ldg(reinterpret_cast<const double2 *>(u)) : make_double2(__ldg(u), __ldg(u + 1));
+    };
+    const double2 b0 = pair(q), b1 = pair(q + ssy), b2 = pair(q + ssz), b3 = pair(q + ssy + ssz);
+    const double a0 = b0.x, a1 = b0.y, a2 = b1.x, a3 = b1.y, a4 = b2.x, a5 = b2.y, a6 = b3.x, a7 = b3.y;
     // order of restrict_3d_cc_rf2.cc:253-260
     double res = mul(w, a0);
     res = madd<FMA>(w, a1, res);
@@ -712,22 +817,74 @@ __device__ __forceinline__ double mono_point(const double *q, int ox, int oy, in
   return res;
 }
 
+// A unit is one coarse base of a fine row, both of its fine points (neighbours
+// in the destination).  Rows are taken by parity, all even fine y before all
+// odd ones and the same in z, so that the threads of a warp evaluate the same
+// stencil (but at the seams) and consecutive lanes consecutive coarse points:
+// point by point in fine order a warp ran every one of its rows' stencils for
+// both x parities.  ns: bases per row.
+__device__ __forceinline__ int by_parity(int m, int n, int s0) { // m-th of 0 .. n-1, those with s0 + x even first
+  const int first = s0 & 1, ne = (n + 1 - first) >> 1; // first even x; how many
+  return m < ne ? first + 2 * m : 1 - first + 2 * (m - ne);
+}
 template <int FMA, int LANES, class D>
 __device__ __forceinline__ void mono_tile(const D &d, int tile, int lid) {
-  constexpr int PER = STILE / LANES;
-  const unsigned npts = (unsigned)d.n[0] * d.n[1] * d.n[2];
-  const unsigned p0 = (unsigned)tile * STILE + lid;
+  constexpr int PER = HTILE / LANES;
+  const unsigned nunits = (unsigned)d.ns * d.n[1] * d.n[2];
+  const unsigned p0 = (unsigned)tile * HTILE + lid;
   const long long sy = d.ssy, sz = d.ssz;
   double *dst = d.dst + (d.doff[0] + d.doff[1] * d.dsy + d.doff[2] * d.dsz);
 #pragma unroll 1
   for (int r = 0; r < PER; ++r) {
     const unsigned p = p0 + r * LANES;
-    if (p >= npts) break;
-    int i, j, k;
-    unflatten(d, p, i, j, k);
-    const int fx = d.soff[0] + i, fy = d.soff[1] + j, fz = d.soff[2] + k;
-    const double *q = d.src[0] + ((fx >> 1) + (fy >> 1) * sy + (long long)(fz >> 1) * sz);
-    dst[i + j * d.dsy + k * d.dsz] = mono_point<FMA>(q, fx & 1, fy & 1, fz & 1, sy, sz);
+    if (p >= nunits) break;
+    const unsigned row = div_magic(p, d.mg[0], d.sh[0]), pl = div_magic(row, d.mg[1], d.sh[1]);
+    const int b = (int)(p - row * (unsigned)d.ns);
+    const int j = by_parity((int)(row - pl * (unsigned)d.n[1]), d.n[1], d.soff[1]);
+    const int k = by_parity((int)pl, d.n[2], d.soff[2]);
+    const int fy = d.soff[1] + j, fz = d.soff[2] + k;
+    const int cx = (d.soff[0] >> 1) + b, i = 2 * cx - d.soff[0]; // the even fine point: -1 .. n[0] - 1
+    const double *q = d.src[0] + (cx + (fy >> 1) * sy + (long long)(fz >> 1) * sz);
+    double *o = dst + (i + j * d.dsy + k * d.dsz);
+    const bool e = i >= 0, f = i + 1 < d.n[0];
+    const double v0 = e ? mono_point<FMA>(q, 0, fy & 1, fz & 1, sy, sz) : 0.0;
+    const double v1 = f ? mono_point<FMA>(q, 1, fy & 1, fz & 1, sy, sz) : 0.0;
+    if (e && f && (reinterpret_cast<uintptr_t>(o) & 15) == 0) {
+      *reinterpret_cast<double2 *>(o) = make_double2(v0, v1);
+    } else {
+      if (e) o[0] = v0;
+      if (f) o[1] = v1;
+    }
+  }
+}
+
+// N source points of a row from q, whose place in 16 bytes `form` gives: 0
+// first, 1 second, 2 unknown (rows of any alignment).  Pairs in one load: the
+// lanes' rows lie 16 bytes apart, so that a load of single points wastes half
+// of every line it touches.
+template <class D> __device__ __forceinline__ int row_form(const D &d, const double *first) {
+  if ((reinterpret_cast<uintptr_t>(d.src[0]) & 15) || (d.ssy & 1) || (d.ssz & 1)) return 2;
+  return (int)((reinterpret_cast<uintptr_t>(first) >> 3) & 1);
+}
+template <int N> __device__ __forceinline__ void load_row(const double *q, int form, double v[N]) {
+  static_assert(N % 2 == 0, "whole pairs");
+  if (form == 0) {
+#pragma unroll
+    for (int m = 0; m < N; m += 2) {
+      const double2 a = __ldg(reinterpret_cast<const double2 *>(q + m));
+      v[m] = a.x;
+      v[m + 1] = a.y;
+    }
+  } else if (form == 1) { // the pairs from one point before to one point after: both in the row's padded length
+#pragma unroll
+    for (int m = -1; m < N; m += 2) {
+      const double2 a = __ldg(reinterpret_cast<const double2 *>(q + m));
+      if (m >= 0) v[m] = a.x;
+      if (m + 1 < N) v[m + 1] = a.y;
+    }
+  } else {
+#pragma unroll
+    for (int m = 0; m < N; ++m) v[m] = __ldg(q + m);
   }
 }
 
@@ -737,12 +894,13 @@ __device__ __forceinline__ void mono_tile(const D &d, int tile, int lid) {
 // fastest; the first term is a plain product.
 template <int FMA, int LANES, class D>
 __device__ __forceinline__ void restrict_cc3_tile(const D &d, int tile, int lid) {
-  constexpr int PER = STILE / LANES;
+  constexpr int PER = HTILE / LANES;
   const unsigned npts = (unsigned)d.n[0] * d.n[1] * d.n[2];
-  const unsigned p0 = (unsigned)tile * STILE + lid;
+  const unsigned p0 = (unsigned)tile * HTILE + lid;
   const long long ssy = d.ssy, ssz = d.ssz;
   const double *s0 = d.src[0] + (d.soff[0] - 1 + (d.soff[1] - 1) * ssy + (d.soff[2] - 1) * ssz);
   double *dst = d.dst + (d.doff[0] + d.doff[1] * d.dsy + d.doff[2] * d.dsz);
+  const int form = row_form(d, s0);
 #pragma unroll 1
   for (int r = 0; r < PER; ++r) {
     const unsigned p = p0 + r * LANES;
@@ -757,13 +915,15 @@ __device__ __forceinline__ void restrict_cc3_tile(const D &d, int tile, int lid)
     for (int c = 0; c < 4; ++c) {
       const double cz = (c == 0 || c == 3) ? -1.0 : 9.0;
       const double *qz = q + c * ssz;
+      double v[4][4];
+#pragma unroll
+      for (int m = 0; m < 4; ++m) load_row<4>(qz + m * ssy, form, v[m]);
       static_for<16>([&](auto M) {
         constexpr int m = decltype(M)::value;
         constexpr double cx = (m & 3) == 0 || (m & 3) == 3 ? -1.0 : 9.0;
         constexpr double cy = (m >> 2) == 0 || (m >> 2) == 3 ? -1.0 : 9.0;
         const double w = cx * cy * cz / 4096.0;
-        const double v = __ldg(qz + (m & 3) + (m >> 2) * ssy);
-        res = (m == 0 && c == 0) ? mul(w, v) : madd<FMA>(w, v, res);
+        res = (m == 0 && c == 0) ? mul(w, v[0][0]) : madd<FMA>(w, v[m >> 2][m & 3], res);
       });
     }
     dst[i + j * d.dsy + k * d.dsz] = res;
@@ -773,12 +933,14 @@ __device__ __forceinline__ void restrict_cc3_tile(const D &d, int tile, int lid)
 // restrict_3d_cc_o5_rf2 (restrict_3d_cc_o5_rf2.cc:36-78): restrict3 over the
 // planes 2k-2 .. 2k+3 of restrict2 over rows of restrict1 over the cells
 // 2i-2 .. 2i+3, each a left-to-right sum with weights (3, -25, 150, 150,
-// -25, 3) / 256, the first term a plain product.
+// -25, 3) / 256, the first term a plain product.  A unit is two coarse points
+// one above the other, which share four of their six planes: each plane's
+// restrict2 is formed once and added to both sums.
 template <int FMA, int LANES, class D>
 __device__ __forceinline__ void restrict_cc5_tile(const D &d, int tile, int lid) {
-  constexpr int PER = STILE / LANES;
-  const unsigned npts = (unsigned)d.n[0] * d.n[1] * d.n[2];
-  const unsigned p0 = (unsigned)tile * STILE + lid;
+  constexpr int PER = HTILE / LANES;
+  const unsigned nunits = (unsigned)d.n[0] * d.n[1] * ((d.n[2] + 1) / 2);
+  const unsigned p0 = (unsigned)tile * HTILE + lid;
   const long long ssy = d.ssy, ssz = d.ssz;
   const double *s0 = d.src[0] + (d.soff[0] - 2 + (d.soff[1] - 2) * ssy + (d.soff[2] - 2) * ssz);
   double *dst = d.dst + (d.doff[0] + d.doff[1] * d.dsy + d.doff[2] * d.dsz);
@@ -786,26 +948,37 @@ __device__ __forceinline__ void restrict_cc5_tile(const D &d, int tile, int lid)
 #pragma unroll 1
   for (int r = 0; r < PER; ++r) {
     const unsigned p = p0 + r * LANES;
-    if (p >= npts) break;
+    if (p >= nunits) break;
     int i, j, k;
     unflatten(d, p, i, j, k);
+    k *= 2;
+    const bool two = k + 1 < d.n[2];
     const double *q = s0 + 2 * (i + j * ssy + k * ssz);
-    double r3 = 0.0;
-#pragma unroll 1
-    for (int c = 0; c < 6; ++c) {
+    const int form = row_form(d, s0);
+    double a0 = 0.0, a1 = 0.0;
+    auto plane = [&](int c) { // restrict2 of plane c of the first point's window
       double r2 = 0.0;
 #pragma unroll
       for (int b = 0; b < 6; ++b) {
-        const double *row = q + c * ssz + b * ssy;
-        double r1 = mul(w[0], __ldg(row));
+        double v[6];
+        load_row<6>(q + c * ssz + b * ssy, form, v);
+        double r1 = mul(w[0], v[0]);
 #pragma unroll
-        for (int a = 1; a < 6; ++a) r1 = madd<FMA>(w[a], __ldg(row + a), r1);
+        for (int a = 1; a < 6; ++a) r1 = madd<FMA>(w[a], v[a], r1);
         r2 = b == 0 ? mul(w[0], r1) : madd<FMA>(w[b], r1, r2);
       }
-      const double wc = (c == 0 || c == 5) ? w[0] : (c == 1 || c == 4) ? w[1] : w[2];
-      r3 = c == 0 ? mul(wc, r2) : madd<FMA>(wc, r2, r3);
+      return r2;
+    };
+    auto weight = [&](int c) { return c == 0 || c == 5 ? w[0] : c == 1 || c == 4 ? w[1] : w[2]; };
+#pragma unroll 1
+    for (int c = 0; c < (two ? 8 : 6); ++c) {
+      const double r2 = plane(c);
+      if (c < 6) a0 = c == 0 ? mul(w[0], r2) : madd<FMA>(weight(c), r2, a0);
+      if (c >= 2) a1 = c == 2 ? mul(w[0], r2) : madd<FMA>(weight(c - 2), r2, a1);
     }
-    dst[i + j * d.dsy + k * d.dsz] = r3;
+    double *o = dst + (i + j * d.dsy + k * d.dsz);
+    o[0] = a0;
+    if (two) o[d.dsz] = a1;
   }
 }
 

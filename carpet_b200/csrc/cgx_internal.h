@@ -60,7 +60,8 @@ constexpr int CONCURRENT_SIDE_MAX = NSEG;
 // (cgx.cu): true when the arrays can be staged by TMA (then maps[0 .. ntl-1]
 // and d.tma are set), false otherwise.
 bool encode_tma_maps(Desc &d, CUtensorMap maps[3]);
-// tiles of a prolongation descriptor in TMA tile configuration `config`
+// tiles of a prolongation descriptor in TMA tile configuration `config` of its
+// variant; those of the cp.async kernels with config < 0
 long long tile_prolongation(Desc &d, int config);
 
 // One plain per-box launch (cgx.cu).
@@ -92,6 +93,15 @@ int klaunch_spair_f1(const Desc &d, int ntiles, int *status, cudaStream_t s);
 CGX_TMA_DECL4(0, 0) CGX_TMA_DECL4(0, 1) CGX_TMA_DECL4(1, 0) CGX_TMA_DECL4(1, 1)
 #undef CGX_TMA_DECL4
 #undef CGX_TMA_DECL
+// the cell-centred ENO families, and single boxes staged by TMA
+int klaunch_tma_eno(int fp, int variant, const Desc *d, const CUtensorMap *maps, const int2 *tmap,
+                    long long ntiles, unsigned long long *counter, int *status, cudaStream_t s);
+#define CGX_BOX_DECL(N) \
+  int klaunch_box_##N(int variant, const Desc &d, const CUtensorMap *maps, int ntiles, int *status, cudaStream_t s);
+CGX_BOX_DECL(f0_p0) CGX_BOX_DECL(f0_p1) CGX_BOX_DECL(f1_p0) CGX_BOX_DECL(f1_p1)
+#undef CGX_BOX_DECL
+int klaunch_box_eno(int fp, int variant, const Desc &d, const CUtensorMap *maps, int ntiles, int *status,
+                    cudaStream_t s);
 int klaunch_stream_f0(int variant, const Desc *d, const int2 *tmap, long long ntiles,
                       unsigned long long *counter, int *status, cudaStream_t s);
 int klaunch_stream_f1(int variant, const Desc *d, const int2 *tmap, long long ntiles,

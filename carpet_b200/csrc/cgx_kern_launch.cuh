@@ -86,7 +86,8 @@ int launch_search_t(const Desc *d_descs, const long long *d_prefix, int ndesc, l
 }
 
 template <int FMA> int launch_spair_t(const Desc &d, int ntiles, int *status, cudaStream_t s) {
-  k_spair<FMA><<<ntiles, NTHREADS, 0, s>>>(d, status);
+  if (d.ns && d.kind == K_COPY) k_spair<FMA, true><<<ntiles, NTHREADS, 0, s>>>(d, status);
+  else k_spair<FMA, false><<<ntiles, NTHREADS, 0, s>>>(d, status);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? CGX_OK : cuda_error(e, "k_spair launch");
 }
@@ -134,6 +135,31 @@ int launch_tma_family(int variant, const Desc *d_descs, const CUtensorMap *d_map
   }
 }
 
+template <int FMA, class F, int NTL, int TK>
+int launch_box_v(const Desc &d, const CUtensorMap *maps, int ntiles, int *status, cudaStream_t s) {
+  static bool attr = false;
+  const size_t smem = sizeof(double) * TSmem<F, NTL, BOX_CFG>::total + 128; // + alignment slack
+  if (!attr) {
+    cudaError_t e = cudaFuncSetAttribute(k_tma_box<FMA, F, NTL, TK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return cuda_error(e, "cudaFuncSetAttribute");
+    attr = true;
+  }
+  BoxMaps m;
+  for (int t = 0; t < 3; ++t) m.m[t] = maps[t];
+  k_tma_box<FMA, F, NTL, TK><<<ntiles, TMA_CFGS[BOX_CFG].nt, smem, s>>>(d, m, status);
+  cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? CGX_OK : cuda_error(e, "k_tma_box launch");
+}
+template <int FMA, class F>
+int launch_box_family(int variant, const Desc &d, const CUtensorMap *maps, int ntiles, int *status, cudaStream_t s) {
+  switch (variant % 4) {
+  case 0: return launch_box_v<FMA, F, 1, T_NONE>(d, maps, ntiles, status, s);
+  case 1: return launch_box_v<FMA, F, 2, T_LIN>(d, maps, ntiles, status, s);
+  case 2: return launch_box_v<FMA, F, 3, T_QUAD>(d, maps, ntiles, status, s);
+  default: return launch_box_v<FMA, F, 3, T_ENO>(d, maps, ntiles, status, s);
+  }
+}
+
 template <int FMA, int V>
 int launch_stream_v(const Desc *d_descs, const int2 *d_tmap, long long ntiles,
                     unsigned long long *d_counter, int *d_status, cudaStream_t s) {
@@ -152,6 +178,10 @@ int launch_stream_map_t(int variant, const Desc *d_descs, const int2 *d_tmap, lo
   case SV_COPY2: return launch_stream_v<FMA, SV_COPY2>(d_descs, d_tmap, ntiles, d_counter, d_status, s);
   case SV_COPY3Q: return launch_stream_v<FMA, SV_COPY3Q>(d_descs, d_tmap, ntiles, d_counter, d_status, s);
   case SV_COPY3E: return launch_stream_v<FMA, SV_COPY3E>(d_descs, d_tmap, ntiles, d_counter, d_status, s);
+  case SV_SECTOR: return launch_stream_v<FMA, SV_SECTOR>(d_descs, d_tmap, ntiles, d_counter, d_status, s);
+  case SV_SECTOR + 1: return launch_stream_v<FMA, SV_SECTOR + 1>(d_descs, d_tmap, ntiles, d_counter, d_status, s);
+  case SV_SECTOR + 2: return launch_stream_v<FMA, SV_SECTOR + 2>(d_descs, d_tmap, ntiles, d_counter, d_status, s);
+  case SV_SECTOR + 3: return launch_stream_v<FMA, SV_SECTOR + 3>(d_descs, d_tmap, ntiles, d_counter, d_status, s);
   case SV_RESTRICT_VC:
     return launch_stream_v<FMA, SV_RESTRICT_VC>(d_descs, d_tmap, ntiles, d_counter, d_status, s);
   case SV_RESTRICT_CC:

@@ -1,5 +1,5 @@
 // cgx_kern_t001.cu -- TMA-staged prolongation kernels, exact mode,
-// families VC<1>, VC<3>, VC<5>, CC<0>, CC<1>, tile configuration 1 (TMA_CFGS).
+// families VC<1>, VC<3>, VC<5>, CC<0>, CC<1>, tile configuration 1 (TMA_CFGS), and their single-box kernels.
 #include "cgx_kern_launch.cuh"
 
 namespace cgx {
@@ -11,6 +11,18 @@ int klaunch_tma_f0_p0_c1(int variant, const Desc *d, const CUtensorMap *maps, co
   case 2: return kern::launch_tma_family<0, VC<5>, 1>(variant, d, maps, tmap, ntiles, counter, status, s);
   case 3: return kern::launch_tma_family<0, CC<0>, 1>(variant, d, maps, tmap, ntiles, counter, status, s);
   case 4: return kern::launch_tma_family<0, CC<1>, 1>(variant, d, maps, tmap, ntiles, counter, status, s);
+  }
+  return set_error(CGX_EINVAL, "bad prolongation variant %d", variant);
+}
+// single boxes (k_tma_box)
+int klaunch_box_f0_p0(int variant, const Desc &d, const CUtensorMap *maps, int ntiles, int *status,
+                      cudaStream_t s) {
+  switch (variant / 4) {
+  case 0: return kern::launch_box_family<0, VC<1>>(variant, d, maps, ntiles, status, s);
+  case 1: return kern::launch_box_family<0, VC<3>>(variant, d, maps, ntiles, status, s);
+  case 2: return kern::launch_box_family<0, VC<5>>(variant, d, maps, ntiles, status, s);
+  case 3: return kern::launch_box_family<0, CC<0>>(variant, d, maps, ntiles, status, s);
+  case 4: return kern::launch_box_family<0, CC<1>>(variant, d, maps, ntiles, status, s);
   }
   return set_error(CGX_EINVAL, "bad prolongation variant %d", variant);
 }

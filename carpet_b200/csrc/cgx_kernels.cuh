@@ -57,6 +57,10 @@ template <int FMA, int NTL, int TK>
 __device__ __noinline__ void copy_entry(const Desc &d, int tile) {
   copy_tile<FMA, NTL, TK, NTHREADS>(d, tile, threadIdx.x);
 }
+template <int FMA, int NTL, int TK>
+__device__ __noinline__ void sectors_entry(const Desc &d, int tile) {
+  copy_sectors<FMA, NTL, TK, NTHREADS>(d, tile, threadIdx.x);
+}
 static __device__ __noinline__ void restrict_vc_entry(const Desc &d, int tile) {
   restrict_vc_tile<NTHREADS>(d, tile, threadIdx.x);
 }
@@ -130,11 +134,16 @@ __device__ __forceinline__ bool run_prolong(const Desc &d, int tile, double *sm)
 template <int FMA> __device__ __forceinline__ void run_tile(const Desc &d, int tile, double *sm, int *status) {
   switch (d.kind) {
   case K_COPY:
-    if (d.ntl == 1) copy_entry<FMA, 1, T_NONE>(d, tile);
-    else if (d.ntl == 2) copy_entry<FMA, 2, T_LIN>(d, tile);
-    else if (d.tkind == T_ENO) copy_entry<FMA, 3, T_ENO>(d, tile);
-    else copy_entry<FMA, 3, T_QUAD>(d, tile);
-    return;
+    switch (stream_variant(d)) {
+    case SV_COPY1: copy_entry<FMA, 1, T_NONE>(d, tile); return;
+    case SV_COPY2: copy_entry<FMA, 2, T_LIN>(d, tile); return;
+    case SV_COPY3Q: copy_entry<FMA, 3, T_QUAD>(d, tile); return;
+    case SV_COPY3E: copy_entry<FMA, 3, T_ENO>(d, tile); return;
+    case SV_SECTOR: sectors_entry<FMA, 1, T_NONE>(d, tile); return;
+    case SV_SECTOR + 1: sectors_entry<FMA, 2, T_LIN>(d, tile); return;
+    case SV_SECTOR + 2: sectors_entry<FMA, 3, T_QUAD>(d, tile); return;
+    default: sectors_entry<FMA, 3, T_ENO>(d, tile); return;
+    }
   case K_RESTRICT_VC: restrict_vc_entry(d, tile); return;
   case K_RESTRICT_CC: restrict_cc_entry<FMA>(d, tile); return;
   case K_RESTRICT_CC3: restrict_cc3_entry<FMA>(d, tile); return;
@@ -149,7 +158,10 @@ __global__ void __launch_bounds__(NTHREADS, HIGH ? 1 : 2)
     k_pair(const __grid_constant__ Desc d, int *status) {
   extern __shared__ __align__(16) double sm[];
   __shared__ __align__(16) Desc s_d;
-  if (threadIdx.x == 0) s_d = d; // field-wise copy out of the parameter space
+  // copied out of the parameter space word by word
+  if (threadIdx.x < sizeof(Desc) / 8)
+    reinterpret_cast<unsigned long long *>(&s_d)[threadIdx.x] =
+        reinterpret_cast<const unsigned long long *>(&d)[threadIdx.x];
   __syncthreads();
   if (!run_prolong<FMA, HIGH, PLAIN_CFG>(s_d, blockIdx.x, sm) && threadIdx.x == 0) report(status, CGX_EDEVICE);
 }
@@ -272,6 +284,10 @@ __device__ __forceinline__ void stream_tile(const Desc &d, int tile, int lid) {
   else if (V == SV_COPY2) copy_tile<FMA, 2, T_LIN, LANES>(d, tile, lid);
   else if (V == SV_COPY3Q) copy_tile<FMA, 3, T_QUAD, LANES>(d, tile, lid);
   else if (V == SV_COPY3E) copy_tile<FMA, 3, T_ENO, LANES>(d, tile, lid);
+  else if (V == SV_SECTOR) copy_sectors<FMA, 1, T_NONE, LANES>(d, tile, lid);
+  else if (V == SV_SECTOR + 1) copy_sectors<FMA, 2, T_LIN, LANES>(d, tile, lid);
+  else if (V == SV_SECTOR + 2) copy_sectors<FMA, 3, T_QUAD, LANES>(d, tile, lid);
+  else if (V == SV_SECTOR + 3) copy_sectors<FMA, 3, T_ENO, LANES>(d, tile, lid);
   else if (V == SV_RESTRICT_VC) restrict_vc_tile<LANES>(d, tile, lid);
   else if (V == SV_RESTRICT_CC) restrict_cc_tile<FMA, LANES>(d, tile, lid);
   else if (V == SV_RESTRICT_CC3) restrict_cc3_tile<FMA, LANES>(d, tile, lid);
@@ -280,27 +296,34 @@ __device__ __forceinline__ void stream_tile(const Desc &d, int tile, int lid) {
   else mono_tile<FMA, LANES>(d, tile, lid);
 }
 
-// Per-box form: a CTA per tile, every variant in one dispatch.  The
-// descriptor parameter is uniform, so its fields are read from the
-// parameter space.
-template <int FMA>
+// Per-box form: a CTA per tile; SECTOR: the copies by sectors, else every
+// other variant in one dispatch.  The descriptor parameter is uniform, so its
+// fields are read from the parameter space.
+template <int FMA, bool SECTOR>
 __global__ void __launch_bounds__(NTHREADS, STREAM_BLOCKS_PER_SM)
     k_spair(const __grid_constant__ Desc d, int *status) {
-  __shared__ __align__(16) Desc s_d;
-  if (threadIdx.x == 0) s_d = d;
-  __syncthreads();
   const int t = blockIdx.x, l = threadIdx.x;
-  switch (stream_variant(s_d)) {
-  case SV_COPY1: stream_tile<FMA, SV_COPY1, NTHREADS>(s_d, t, l); return;
-  case SV_COPY2: stream_tile<FMA, SV_COPY2, NTHREADS>(s_d, t, l); return;
-  case SV_COPY3Q: stream_tile<FMA, SV_COPY3Q, NTHREADS>(s_d, t, l); return;
-  case SV_COPY3E: stream_tile<FMA, SV_COPY3E, NTHREADS>(s_d, t, l); return;
-  case SV_RESTRICT_VC: stream_tile<FMA, SV_RESTRICT_VC, NTHREADS>(s_d, t, l); return;
-  case SV_RESTRICT_CC: stream_tile<FMA, SV_RESTRICT_CC, NTHREADS>(s_d, t, l); return;
-  case SV_RESTRICT_CC3: stream_tile<FMA, SV_RESTRICT_CC3, NTHREADS>(s_d, t, l); return;
-  case SV_RESTRICT_CC5: stream_tile<FMA, SV_RESTRICT_CC5, NTHREADS>(s_d, t, l); return;
-  case SV_TIME: stream_tile<FMA, SV_TIME, NTHREADS>(s_d, t, l); return;
-  case SV_MONO: stream_tile<FMA, SV_MONO, NTHREADS>(s_d, t, l); return;
+  if constexpr (SECTOR) {
+    switch (stream_variant(d)) {
+    case SV_SECTOR: stream_tile<FMA, SV_SECTOR, NTHREADS>(d, t, l); return;
+    case SV_SECTOR + 1: stream_tile<FMA, SV_SECTOR + 1, NTHREADS>(d, t, l); return;
+    case SV_SECTOR + 2: stream_tile<FMA, SV_SECTOR + 2, NTHREADS>(d, t, l); return;
+    case SV_SECTOR + 3: stream_tile<FMA, SV_SECTOR + 3, NTHREADS>(d, t, l); return;
+    }
+    if (threadIdx.x == 0) report(status, CGX_EDEVICE);
+    return;
+  }
+  switch (stream_variant(d)) {
+  case SV_COPY1: stream_tile<FMA, SV_COPY1, NTHREADS>(d, t, l); return;
+  case SV_COPY2: stream_tile<FMA, SV_COPY2, NTHREADS>(d, t, l); return;
+  case SV_COPY3Q: stream_tile<FMA, SV_COPY3Q, NTHREADS>(d, t, l); return;
+  case SV_COPY3E: stream_tile<FMA, SV_COPY3E, NTHREADS>(d, t, l); return;
+  case SV_RESTRICT_VC: stream_tile<FMA, SV_RESTRICT_VC, NTHREADS>(d, t, l); return;
+  case SV_RESTRICT_CC: stream_tile<FMA, SV_RESTRICT_CC, NTHREADS>(d, t, l); return;
+  case SV_RESTRICT_CC3: stream_tile<FMA, SV_RESTRICT_CC3, NTHREADS>(d, t, l); return;
+  case SV_RESTRICT_CC5: stream_tile<FMA, SV_RESTRICT_CC5, NTHREADS>(d, t, l); return;
+  case SV_TIME: stream_tile<FMA, SV_TIME, NTHREADS>(d, t, l); return;
+  case SV_MONO: stream_tile<FMA, SV_MONO, NTHREADS>(d, t, l); return;
   }
   if (threadIdx.x == 0) report(status, CGX_EDEVICE);
 }
@@ -411,6 +434,28 @@ __global__ void __launch_bounds__(TMA_CFGS[CFG].nt, tma_blocks<F, NTL, TK, CFG>(
     }
     __syncthreads();
   }
+}
+
+// One box-pair staged by TMA, a CTA per tile: the plain per-box form where the
+// source arrays can be described to the tensor-copy unit (the tensor maps
+// travel as kernel parameters).
+struct BoxMaps {
+  CUtensorMap m[3];
+};
+template <int FMA, class F, int NTL, int TK>
+__global__ void __launch_bounds__(TMA_CFGS[BOX_CFG].nt, tma_blocks<F, NTL, TK, BOX_CFG>())
+    k_tma_box(const __grid_constant__ Desc d, const __grid_constant__ BoxMaps maps, int *status) {
+  extern __shared__ __align__(128) double smraw[];
+  const unsigned sbase = smem_u32(smraw);
+  double *sm = smraw + ((((sbase + 127u) & ~127u) - sbase) >> 3);
+  __shared__ __align__(8) uint64_t s_bars[TMA_NB];
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < TMA_NB; ++i) mbar_init(&s_bars[i], 1);
+    mbar_fence_init();
+  }
+  __syncthreads();
+  TmaRing ring{s_bars};
+  prolong_tile<F, FMA, NTL, TK, BOX_CFG, true>(d, maps.m, (int)blockIdx.x, sm, ring, status);
 }
 
 // dynamic shared memory of the widest variant a kernel dispatches

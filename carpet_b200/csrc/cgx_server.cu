@@ -541,7 +541,7 @@ int cgx_server_define_op(cgx_server *sv, int hier, const cgx_batch *pairs, int *
       pd[i] = t;
       pnt[i] = tn;
     } else {
-      pd[i].tma = 0;
+      pnt[i] = tile_prolongation(pd[i], -1);
     }
   }
   for (int i = 0; i < n; ++i) {
@@ -581,7 +581,7 @@ int cgx_server_define_op(cgx_server *sv, int hier, const cgx_batch *pairs, int *
 }
 
 int cgx_server_set_config(cgx_server *sv, int variant, int config) {
-  if (!sv || variant < -1 || variant >= TV_COUNT || config < 0 || config >= TMA_NCFG)
+  if (!sv || variant < -1 || variant >= TV_TUNED || config < 0 || config >= TMA_NCFG)
     return set_error(CGX_EINVAL, "server set_config: variant %d / configuration %d out of range", variant,
                      config);
   std::lock_guard<std::mutex> dg(sv->define_mu);

@@ -49,8 +49,9 @@ struct TmaCfg {
 constexpr TmaCfg TMA_CFGS[] = {{256, 16, 64, 2}, {128, 8, 64, 4}, {128, 8, 32, 4}, {128, 8, 64, 5}, {128, 8, 32, 6}};
 constexpr int TMA_NCFG = 5;
 constexpr int tma_kernel_cfg(int c) { return c == 2 ? 1 : c; }
-// the configuration of the kernels that stage by cp.async
-constexpr int PLAIN_CFG = 0;
+// the configuration of the kernels that stage by cp.async, and that of a
+// single box staged by TMA
+constexpr int PLAIN_CFG = 0, BOX_CFG = 1;
 // mbarriers per CTA: one per stage slot
 constexpr int TMA_NB = 2;
 
@@ -110,15 +111,21 @@ template <class F, int NTL, int TK, int CFG> constexpr int tma_blocks() {
   return b < 1 ? 1 : b > 1024 / NT ? 1024 / NT : b;
 }
 
-// The TMA kernels' variants: family (VC 1/3/5, CC 0-5, ENO) x time
-// interpolation (one timelevel, linear, quadratic, ENO).
-constexpr int TV_FAMILIES = 10;
+// The TMA kernels' variants: family (VC 1/3/5, CC 0-5, ENO; cell-centred ENO
+// 2/3) x time interpolation (one timelevel, linear, quadratic, ENO).  The
+// first TV_TUNED have a kernel per tile configuration; the cell-centred ENO
+// ones run in TV_FIXED_CFG.
+constexpr int TV_TUNED = 40;
+constexpr int TV_FAMILIES = 12;
 constexpr int TV_COUNT = 4 * TV_FAMILIES;
+constexpr int TV_FIXED_CFG = 1;
+constexpr int tma_cfg(int variant, int cfg) { return variant < TV_TUNED ? cfg : TV_FIXED_CFG; }
 template <class D> __host__ __device__ __forceinline__ int tma_variant(const D &d) {
   int f = -1;
   if (d.kind == K_PROLONG_VC) f = d.order == 1 ? 0 : d.order == 3 ? 1 : d.order == 5 ? 2 : -1;
   else if (d.kind == K_PROLONG_CC) f = d.order >= 0 && d.order <= 5 ? 3 + d.order : -1;
   else if (d.kind == K_PROLONG_ENO) f = 9;
+  else if (d.kind == K_PROLONG_CC_ENO) f = d.order == 2 ? 10 : d.order == 3 ? 11 : -1;
   if (f < 0) return -1;
   const int tv = d.ntl == 1 ? 0 : d.ntl == 2 ? 1 : d.tkind == T_ENO ? 3 : 2;
   return 4 * f + tv;
