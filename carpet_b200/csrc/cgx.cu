@@ -1226,6 +1226,12 @@ int cgx_batch_upload(cgx_batch *b, void *stream) {
   if (8 * narrow > copied)
     for (int i : order)
       if (dq[i].kind == K_COPY && dq[i].ns) ntq[i] = stream_tiles(dq[i], 0);
+  // Batches that copy more than L2 keeps fetch their destinations ahead: a
+  // ghost sync of 25 grid functions of 129^3 (125 MB) 76.2 -> 72.0 us and the
+  // five-level step, whose syncs of 60 MB each find nothing in L2,
+  // 7.54 -> 7.24 ms; a sync of 8 (40 MB), its arrays in L2, took 22.0 instead
+  // of 20.6 us.
+  for (int i : order) dq[i].ahead = dq[i].kind == K_COPY && 16 * copied >= 48 << 20;
   for (const auto &kv : by_variant) {
     const int cfg = kv.first >= 0 ? tma_cfg(kv.first, b->tma_cfg[kv.first]) : PLAIN_CFG;
     PzCost cost(cfg);

@@ -59,7 +59,7 @@ struct Desc {
   unsigned char xo, xw;
   short pz; // fine z points of a tile (even)
   unsigned char xs2;
-  unsigned char pad0;
+  unsigned char ahead; // copies: fetch the destination with the sources
   int rpx; // ceil(65536 / ptx): t / ptx = t * rpx >> 16 for t < 256
   int ns;  // copies: units per row (Sector), 0: point by point; monotone prolongation: coarse bases per row
   long long ssy, ssz; // source strides (elements) in y and z
@@ -492,11 +492,6 @@ __device__ __forceinline__ void unflatten(const D &d, unsigned p, int &i, int &j
   k = (int)r;
 }
 
-// group sizes: points whose loads a thread issues before it stores them
-template <int LANES, int NTL> __host__ __device__ constexpr int stream_group() {
-  return (STILE / LANES) < (NTL == 1 ? 8 : 4) ? (STILE / LANES) : (NTL == 1 ? 8 : 4);
-}
-
 // Unit p of the region's destination rows, the rows' first and last sectors
 // whole: its row, and the x (-7 .. n[0] + 6) of its first half sector, which
 // starts on 16 bytes; the other half lies four points further.
@@ -590,6 +585,10 @@ __device__ __forceinline__ void copy_tile(const D &d, int tile, int lid) {
   constexpr int G = G0 / (TK == T_ENO ? 2 : 1);
   const unsigned npts = (unsigned)d.n[0] * d.n[1] * d.n[2];
   const unsigned p0 = (unsigned)tile * PTS + lid;
+  // the pieces of a row that a warp stores start and end inside sectors, whose
+  // rest L2 fetches from DRAM as the store arrives: the destination fetched
+  // with the sources instead
+  const bool ahead = d.ahead;
   const double *src[NTL];
 #pragma unroll
   for (int t = 0; t < NTL; ++t) src[t] = d.src[t] + (d.soff[0] + d.soff[1] * d.ssy + d.soff[2] * d.ssz);
@@ -609,6 +608,7 @@ __device__ __forceinline__ void copy_tile(const D &d, int tile, int lid) {
         const long long si = i + j * d.ssy + k * d.ssz;
 #pragma unroll
         for (int t = 0; t < NTL; ++t) v[r][t] = ld_src<CG>(src[t] + si);
+        if (ahead) asm volatile("prefetch.global.L2 [%0];" ::"l"(dst + (i + j * d.dsy + k * d.dsz)));
       }
     }
     // the destination index is recomputed rather than held across the loads
