@@ -76,7 +76,7 @@ struct Box {
 
 // The magic number and shift of div_magic (cgx_device.cuh) for divisor n:
 // l = ceil(log2 n), m = ceil(2^(31+l) / n), s = l - 1; m = 0 encodes n = 1.
-void division_magic(int n, unsigned *m, int *s) {
+void division_magic(int n, unsigned *m, unsigned char *s) {
   if (n <= 1) {
     *m = 0;
     *s = 0;
@@ -86,7 +86,7 @@ void division_magic(int n, unsigned *m, int *s) {
   while ((1LL << l) < n) ++l;
   const unsigned long long num = 1ULL << (31 + l); // l <= 31
   *m = (unsigned)((num + (unsigned)n - 1) / (unsigned)n);
-  *s = l - 1;
+  *s = (unsigned char)(l - 1);
 }
 
 struct Win { int lo0, hi0, lo1, hi1; };

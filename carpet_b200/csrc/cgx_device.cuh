@@ -44,8 +44,11 @@ constexpr int NWARPS = NTHREADS / 32;
 // planes.  The shape is chosen per descriptor (prolong_tiles in cgx.cu).
 constexpr int PTXMAX = 16;
 
+// 224 bytes: as a kernel parameter with a pointer beside it, a descriptor of 8
+// bytes more costs each per-box launch 0.35 us of the host's time (2.30 against
+// 2.67 us a launch, parameters of up to 232 bytes and of more).
 struct Desc {
-  int kind, order, ntl, tkind;
+  unsigned char kind, order, ntl, tkind;
   int n[3];     // destination region extent (points)
   int soff[3];  // source offset of the region start (meaning per kind)
   int doff[3];  // destination index of the region start
@@ -62,14 +65,15 @@ struct Desc {
   unsigned char ahead; // copies: fetch the destination with the sources
   int rpx; // ceil(65536 / ptx): t / ptx = t * rpx >> 16 for t < 256
   int ns;  // copies: units per row (Sector), 0: point by point; monotone prolongation: coarse bases per row
+  unsigned char sh[2]; // division magic (div_magic) for ns or n[0], n[1]; prolongation: tiles[0], tiles[1]
+  unsigned mg[2];
   long long ssy, ssz; // source strides (elements) in y and z
   long long dsy, dsz; // destination strides
-  unsigned mg[2]; // division magic (div_magic) for ns or n[0], n[1]; prolongation: tiles[0], tiles[1]
-  int sh[2];
   const double *src[3];
   double *dst;
   double w[8]; // time weights (layout of the oracle's cgxo_time_weights)
 };
+static_assert(sizeof(Desc) == 224, "descriptor size");
 
 // compile-time loop: f(std::integral_constant<int, 0>()) ... f(<N-1>)
 template <class Fn, int... I>
