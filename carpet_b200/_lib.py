@@ -44,6 +44,8 @@ _i3 = C.c_int * 3
 lib.cgx_transfer.argtypes = [C.c_int, C.c_int, _P(cgx_array), _P(cgx_array), _P(C.c_double),
                              C.c_int, _i9, _i9, C.c_void_p, C.c_double, C.c_int, C.c_int,
                              C.c_void_p]
+# a cgx_pair record, packed by carpet_b200.transfer
+lib.cgx_transfer_pair.argtypes = [C.c_char_p, C.c_void_p]
 lib.cgx_copy.argtypes = [C.c_int, C.c_int, _P(cgx_array), _P(cgx_array), _i9, _i9, C.c_void_p,
                          C.c_void_p]
 lib.cgx_batch_add.argtypes = [C.c_void_p, C.c_int, C.c_int, _P(cgx_array), _P(cgx_array),

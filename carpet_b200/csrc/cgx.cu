@@ -1069,6 +1069,13 @@ int cgx_transfer(int op, int cent, const cgx_array *dst, const cgx_array *srcs, 
   return launch_pair(b.d, b.ntiles, g_fp_mode, nullptr, (cudaStream_t)stream);
 }
 
+int cgx_transfer_pair(const cgx_pair *p, void *stream) {
+  if (!p) return fail(CGX_EINVAL, "transfer: null argument");
+  if (p->nsrc > 3) return fail(CGX_EINVAL, "transfer: a record holds at most 3 source timelevels");
+  return cgx_transfer(p->op, p->cent, &p->dst, p->srcs, p->times, p->nsrc, p->dstbox, p->srcbox,
+                      p->has_slab ? p->slab_offset : nullptr, p->time, p->order_space, p->order_time, stream);
+}
+
 int cgx_copy(int op, int cent, const cgx_array *dst, const cgx_array *src, const int dstbox[9],
              const int srcbox[9], const int *slab_offset, void *stream) {
   // gdata::copy_data, gdata.cc:110-122

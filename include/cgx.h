@@ -405,6 +405,10 @@ typedef struct cgx_pair {
   int order_space, order_time;
 } cgx_pair;
 int cgx_transfer_pairs_noalloc(const cgx_pair *pairs, int npairs, void *stream);
+/* cgx_transfer of one box-pair given as a record (at most 3 source
+ * timelevels), for bindings whose cost per argument counts: same checks, same
+ * launch. */
+int cgx_transfer_pair(const cgx_pair *pair, void *stream);
 /* Waits for the stream and returns the status the last
  * cgx_transfer_pairs_noalloc kernel on the current device left in the fixed
  * scratch: CGX_OK, or CGX_EDEVICE when a bounded device wait gave up.
