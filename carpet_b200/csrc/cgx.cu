@@ -286,7 +286,7 @@ bool tma_addressable(const Desc &d) {
 // (cgx_device.cuh).  ns: a copy's units per row, or 0.
 long long stream_tiles(Desc &d, int ns) {
   if ((long long)d.n[0] * d.n[1] * d.n[2] >= (1LL << 31)) return -1;
-  long long row = d.n[0], planes = d.n[2];
+  long long row = d.n[0];
   int per = STILE;
   d.ns = ns;
   if (ns) {
@@ -298,10 +298,13 @@ long long stream_tiles(Desc &d, int ns) {
   } else if (d.kind == K_RESTRICT_CC || d.kind == K_RESTRICT_CC3) {
     per = HTILE;
   } else if (d.kind == K_RESTRICT_CC5) {
-    planes = (planes + 1) / 2;
-    per = HTILE;
+    d.tiles[0] = ceil_div(d.n[0], CC5X);
+    d.tiles[1] = ceil_div(d.n[1], CC5Y);
+    d.pz = (long long)d.n[0] * d.n[1] * d.n[2] >= 1 << 16 ? 16 : 4;
+    d.tiles[2] = ceil_div(d.n[2], d.pz);
+    return (long long)d.tiles[0] * d.tiles[1] * d.tiles[2];
   }
-  d.tiles[0] = (int)((row * d.n[1] * planes + per - 1) / per);
+  d.tiles[0] = (int)((row * d.n[1] * d.n[2] + per - 1) / per);
   d.tiles[1] = d.tiles[2] = 1;
   division_magic((int)row, &d.mg[0], &d.sh[0]);
   division_magic(d.n[1], &d.mg[1], &d.sh[1]);

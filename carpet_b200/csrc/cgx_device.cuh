@@ -937,52 +937,81 @@ __device__ __forceinline__ void restrict_cc3_tile(const D &d, int tile, int lid)
 // restrict_3d_cc_o5_rf2 (restrict_3d_cc_o5_rf2.cc:36-78): restrict3 over the
 // planes 2k-2 .. 2k+3 of restrict2 over rows of restrict1 over the cells
 // 2i-2 .. 2i+3, each a left-to-right sum with weights (3, -25, 150, 150,
-// -25, 3) / 256, the first term a plain product.  A unit is two coarse points
-// one above the other, which share four of their six planes: each plane's
-// restrict2 is formed once and added to both sums.
+// -25, 3) / 256, the first term a plain product.  The CTA marches a tile of
+// CC5X x CC5Y x pz coarse points plane by plane: restrict1 of the plane's
+// rows into shared memory, restrict2 by the column's thread, which adds it to
+// the three sums that the plane belongs to.  Every value is formed once per
+// tile: about 100 operations and 30 loads of 16 bytes a point, where a point on
+// its own takes 473 and 108 and was bound by L1 (96 uneven regions of 8-32
+// coarse points a side: 246 us, two points sharing planes 103 us, this form
+// 57 us; beside the other restrictions of such a batch 189 -> 59 us in all).
+// Small regions take short tiles (pz 4), which run at once; large ones 16,
+// with fewer halo planes.
+constexpr int CC5X = 16, CC5Y = 8;
 template <int FMA, int LANES, class D>
 __device__ __forceinline__ void restrict_cc5_tile(const D &d, int tile, int lid) {
-  constexpr int PER = HTILE / LANES;
-  const unsigned nunits = (unsigned)d.n[0] * d.n[1] * ((d.n[2] + 1) / 2);
-  const unsigned p0 = (unsigned)tile * HTILE + lid;
+  constexpr int ROWS = 2 * CC5Y + 4;
+  static_assert(CC5X * CC5Y <= LANES, "a thread per column");
+  __shared__ double r1[2][ROWS * CC5X];
+  const int tx = tile % d.tiles[0], rr = tile / d.tiles[0], ty = rr % d.tiles[1], tz = rr / d.tiles[1];
+  const int i0 = tx * CC5X, j0 = ty * CC5Y, k0 = tz * d.pz;
+  const int nx = min(CC5X, d.n[0] - i0), ny = min(CC5Y, d.n[1] - j0), nz = min((int)d.pz, d.n[2] - k0);
   const long long ssy = d.ssy, ssz = d.ssz;
-  const double *s0 = d.src[0] + (d.soff[0] - 2 + (d.soff[1] - 2) * ssy + (d.soff[2] - 2) * ssz);
-  double *dst = d.dst + (d.doff[0] + d.doff[1] * d.dsy + d.doff[2] * d.dsz);
+  const double *s0 = d.src[0] + (d.soff[0] - 2 + 2 * i0 + (d.soff[1] - 2 + 2 * j0) * ssy + (d.soff[2] - 2 + 2 * k0) * ssz);
   constexpr double w[6] = {3.0 / 256, -25.0 / 256, 150.0 / 256, 150.0 / 256, -25.0 / 256, 3.0 / 256};
-#pragma unroll 1
-  for (int r = 0; r < PER; ++r) {
-    const unsigned p = p0 + r * LANES;
-    if (p >= nunits) break;
-    int i, j, k;
-    unflatten(d, p, i, j, k);
-    k *= 2;
-    const bool two = k + 1 < d.n[2];
-    const double *q = s0 + 2 * (i + j * ssy + k * ssz);
-    const int form = row_form(d, s0);
-    double a0 = 0.0, a1 = 0.0;
-    auto plane = [&](int c) { // restrict2 of plane c of the first point's window
-      double r2 = 0.0;
+  const int form = row_form(d, s0);
+  const int i = lid % CC5X, j = lid / CC5X;
+  const bool owner = i < nx && j < ny;
+  double *out = d.dst + (d.doff[0] + i0 + i + (d.doff[1] + j0 + j) * d.dsy + (d.doff[2] + k0) * d.dsz);
+  // the thread's rows of a plane; those of the next plane are loaded before the
+  // barrier, so that a plane costs no memory latency of its own
+  constexpr int STEP = LANES / CC5X, R = (ROWS + STEP - 1) / STEP;
+  const int rows = i < nx ? 2 * ny + 4 : 0, planes = 2 * nz + 4;
+  double v[R][6];
+  auto fetch = [&](int c) {
 #pragma unroll
-      for (int b = 0; b < 6; ++b) {
-        double v[6];
-        load_row<6>(q + c * ssz + b * ssy, form, v);
-        double r1 = mul(w[0], v[0]);
+    for (int r = 0; r < R; ++r)
+      if (j + r * STEP < rows) load_row<6>(s0 + 2 * i + (j + r * STEP) * ssy + c * ssz, form, v[r]);
+  };
+  fetch(0);
+  auto plane = [&](int c) { // restrict2 of plane c of the tile
+    double *buf = r1[c & 1];
 #pragma unroll
-        for (int a = 1; a < 6; ++a) r1 = madd<FMA>(w[a], v[a], r1);
-        r2 = b == 0 ? mul(w[0], r1) : madd<FMA>(w[b], r1, r2);
+    for (int r = 0; r < R; ++r)
+      if (j + r * STEP < rows) {
+        double x = mul(w[0], v[r][0]);
+#pragma unroll
+        for (int a = 1; a < 6; ++a) x = madd<FMA>(w[a], v[r][a], x);
+        buf[(j + r * STEP) * CC5X + i] = x;
       }
-      return r2;
-    };
-    auto weight = [&](int c) { return c == 0 || c == 5 ? w[0] : c == 1 || c == 4 ? w[1] : w[2]; };
-#pragma unroll 1
-    for (int c = 0; c < (two ? 8 : 6); ++c) {
-      const double r2 = plane(c);
-      if (c < 6) a0 = c == 0 ? mul(w[0], r2) : madd<FMA>(weight(c), r2, a0);
-      if (c >= 2) a1 = c == 2 ? mul(w[0], r2) : madd<FMA>(weight(c - 2), r2, a1);
+    if (c + 1 < planes) fetch(c + 1);
+    __syncthreads();
+    double r2 = 0.0;
+    if (owner) {
+      const double *col = buf + 2 * j * CC5X + i;
+      r2 = mul(w[0], col[0]);
+#pragma unroll
+      for (int b = 1; b < 6; ++b) r2 = madd<FMA>(w[b], col[b * CC5X], r2);
     }
-    double *o = dst + (i + j * d.dsy + k * d.dsz);
-    o[0] = a0;
-    if (two) o[d.dsz] = a1;
+    return r2;
+  };
+  double a0 = 0.0, a1 = 0.0, a2 = 0.0; // the sums of points m, m - 1, m - 2
+#pragma unroll 1
+  for (int m = 0; m < nz + 2; ++m) {
+    double r2 = plane(2 * m);
+    a0 = mul(w[0], r2);
+    a1 = madd<FMA>(w[2], r2, a1);
+    a2 = madd<FMA>(w[4], r2, a2);
+    r2 = plane(2 * m + 1);
+    a0 = madd<FMA>(w[1], r2, a0);
+    a1 = madd<FMA>(w[3], r2, a1);
+    a2 = madd<FMA>(w[5], r2, a2);
+    if (m >= 2) {
+      if (owner) *out = a2;
+      out += d.dsz;
+    }
+    a2 = a1;
+    a1 = a0;
   }
 }
 

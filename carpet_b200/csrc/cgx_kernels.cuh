@@ -274,7 +274,9 @@ __global__ void __launch_bounds__(NTHREADS, 2)
 // they run at high occupancy -- many warps keep their loads in flight.
 constexpr int STREAM_BLOCKS_PER_SM = 4;
 // the persistent streaming kernels: smaller CTAs, more of them per SM
-constexpr int STREAM_THREADS = 128, STREAM_MAP_BLOCKS_PER_SM = 8;
+constexpr int STREAM_THREADS = 128;
+// the fifth-order restriction holds the values of the next plane's rows
+__host__ __device__ constexpr int stream_blocks(int v) { return v == SV_RESTRICT_CC5 ? 6 : 8; }
 
 // one streaming variant's tile, run by LANES threads (lid: 0 .. LANES-1);
 // V is a StreamVariant
@@ -334,7 +336,7 @@ __global__ void __launch_bounds__(NTHREADS, STREAM_BLOCKS_PER_SM)
 // tile's descriptor into the second of two shared buffers while the current
 // tile runs.
 template <int FMA, int V>
-__global__ void __launch_bounds__(STREAM_THREADS, STREAM_MAP_BLOCKS_PER_SM)
+__global__ void __launch_bounds__(STREAM_THREADS, stream_blocks(V))
     k_stream_map(const Desc *__restrict__ descs, const int2 *__restrict__ tmap, long long ntiles,
                  unsigned long long *counter, int *status) {
   __shared__ __align__(16) Desc s_d[2];
