@@ -1906,7 +1906,7 @@ namespace cgx {
 int launch_map_concurrent(int fp, const Desc *d, const CUtensorMap *maps, const int2 *tmap,
                           const long long seg[NSEG + 1], const int *cfg, unsigned long long *counter,
                           int *status, cudaStream_t s, const cudaStream_t *side, const cudaEvent_t *ev,
-                          int nside_have, int *need, const int *caps) {
+                          int nside_have, int *need, const int *caps, bool share) {
   constexpr int TSEG = SEG_STREAM + SV_TIME;
   static_assert(TSEG == NSEG - 1, "the time combination is the last segment");
   int idx[NSEG], n = 0;
@@ -1914,8 +1914,8 @@ int launch_map_concurrent(int fp, const Desc *d, const CUtensorMap *maps, const 
     if (seg[i + 1] > seg[i]) idx[n++] = i;
   *need = 0;
   if (n <= 1) return launch_map(fp, d, maps, tmap, seg, cfg, counter, status, s, caps);
-  const int nside = n - 1;
-  if (nside_have < nside) {
+  const int nside = share ? std::min(n - 1, nside_have) : n - 1;
+  if (nside_have < nside || nside < 1) {
     *need = nside;
     return fail(CGX_EINVAL, "concurrent launch: %d side streams needed, %d given", nside, nside_have);
   }
@@ -1935,7 +1935,7 @@ int launch_map_concurrent(int fp, const Desc *d, const CUtensorMap *maps, const 
   for (int j = 0; j < n && rc == CGX_OK; ++j) {
     long long sg[NSEG + 1];
     only(idx[j], sg);
-    rc = launch_map(fp, d, maps, tmap, sg, cfg, counter, status, j == 0 ? s : side[j - 1], caps);
+    rc = launch_map(fp, d, maps, tmap, sg, cfg, counter, status, j == 0 ? s : side[(j - 1) % nside], caps);
   }
   // join every forked side stream, also after a failure
   cudaError_t je = cudaSuccess;
@@ -2001,6 +2001,8 @@ long long tile_prolongation(Desc &d, int config) {
   const int c = config < 0 ? PLAIN_CFG : tma_cfg(tma_variant(d), config);
   return prolong_tiles(d, c, TMA_CFGS[c].pz);
 }
+
+long long tile_points(Desc &d) { return stream_tiles(d, 0); }
 
 bool encode_tma_maps(Desc &d, CUtensorMap maps[3]) {
   if (!tma_addressable(d)) return false;

@@ -48,13 +48,15 @@ int launch_tile_map(const Desc *d_descs, const CUtensorMap *d_maps, const int2 *
 // The segments of a tile map launched concurrently (cgx.cu): every
 // non-empty segment but the time combination on a stream of its own
 // (side[0 .. nside-1], forked from s with ev[0] and joined back with
-// ev[1 + k]), then the time segment on s; nside + 1 events.  Returns the
-// number of side streams needed in *need when they do not suffice.
+// ev[1 + k]), then the time segment on s; nside + 1 events.  With fewer side
+// streams than segments: with `share`, segments share them (one after another
+// on a stream); else the call fails and *need is the number needed.
 int launch_map_concurrent(int fp, const Desc *d, const CUtensorMap *maps, const int2 *tmap,
                           const long long seg[NSEG + 1], const int *cfg, unsigned long long *counter,
                           int *status, cudaStream_t s, const cudaStream_t *side, const cudaEvent_t *ev,
-                          int nside, int *need, const int *caps = nullptr);
-constexpr int CONCURRENT_SIDE_MAX = NSEG;
+                          int nside, int *need, const int *caps = nullptr, bool share = false);
+// side streams of a server slot (a served launch has a handful of segments)
+constexpr int SERVER_SIDE = 24;
 
 // The tensor maps of a tiled prolongation descriptor's source timelevels
 // (cgx.cu): true when the arrays can be staged by TMA (then maps[0 .. ntl-1]
@@ -63,6 +65,8 @@ bool encode_tma_maps(Desc &d, CUtensorMap maps[3]);
 // tiles of a prolongation descriptor in TMA tile configuration `config` of its
 // variant; those of the cp.async kernels with config < 0
 long long tile_prolongation(Desc &d, int config);
+// tiles of a copy that goes point by point whatever its rows' width
+long long tile_points(Desc &d);
 
 // One plain per-box launch (cgx.cu).
 int launch_one_pair(const Desc &d, int ntiles, int fp, int *status, cudaStream_t s);

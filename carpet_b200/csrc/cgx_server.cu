@@ -79,8 +79,8 @@ struct Slot {
   // read back (the worker retires the slot on it, sleeping if it must)
   cudaEvent_t done = nullptr, fin = nullptr;
   // the concurrent segment launch: side streams, fork and join events
-  cudaStream_t side[CONCURRENT_SIDE_MAX] = {};
-  cudaEvent_t ev[CONCURRENT_SIDE_MAX + 1] = {};
+  cudaStream_t side[SERVER_SIDE] = {};
+  cudaEvent_t ev[SERVER_SIDE + 1] = {};
   int2 *d_tmap = nullptr, *h_tmap = nullptr;
   unsigned long long *d_counter = nullptr;
   // the launch's device status (a bounded wait that gave up: CGX_EDEVICE),
@@ -172,9 +172,9 @@ int slot_init(Slot &s, size_t tile_cap) {
   if (e == cudaSuccess) e = cudaMemset(s.d_status, 0, sizeof(int));
   if (e == cudaSuccess) e = cudaMallocHost(&s.h_status, sizeof(int));
   if (e == cudaSuccess) *s.h_status = 0;
-  for (int k = 0; k < CONCURRENT_SIDE_MAX && e == cudaSuccess; ++k)
+  for (int k = 0; k < SERVER_SIDE && e == cudaSuccess; ++k)
     e = cudaStreamCreateWithFlags(&s.side[k], cudaStreamNonBlocking);
-  for (int k = 0; k <= CONCURRENT_SIDE_MAX && e == cudaSuccess; ++k)
+  for (int k = 0; k <= SERVER_SIDE && e == cudaSuccess; ++k)
     e = cudaEventCreateWithFlags(&s.ev[k], cudaEventDisableTiming);
   if (e != cudaSuccess) return cuda_error(e, "server slot allocation");
   s.tile_cap = tile_cap;
@@ -333,7 +333,7 @@ bool launch_batch(cgx_server *sv, int slot) {
   if (rc == CGX_OK && seg[NSEG] > 0) {
     int need = 0;
     rc = launch_map_concurrent(sv->fp, pdescs, pmaps, s.d_tmap, seg, sv->tma_cfg, s.d_counter, s.d_status,
-                               s.stream, s.side, s.ev, CONCURRENT_SIDE_MAX, &need);
+                               s.stream, s.side, s.ev, SERVER_SIDE, &need, nullptr, true);
   }
   note_error(sv, rc);
   e = cudaEventRecord(s.done, s.stream);
@@ -532,6 +532,9 @@ int cgx_server_define_op(cgx_server *sv, int hier, const cgx_batch *pairs, int *
   std::vector<long long> pnt(nt, nt + n);
   std::vector<CUtensorMap> maps(3 * (size_t)n);
   for (int i = 0; i < n; ++i) {
+    // copies go point by point, one kernel for narrow and wide rows: a launch
+    // of small hierarchies costs the worker more in kernels than the GPU in time
+    if (pd[i].kind == K_COPY && pd[i].ns) pnt[i] = tile_points(pd[i]);
     if (!is_stencil(pd[i].kind)) continue;
     const int v = tma_variant(pd[i]);
     Desc t = pd[i];
