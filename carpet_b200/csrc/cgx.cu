@@ -450,7 +450,7 @@ struct Built {
   int ntiles;
   int nst;            // timelevels staged through temporaries, or 0
   Desc st[5];
-  int st_ntiles;
+  int st_ntiles[5];   // each stage its own: timelevels may be staged in different forms
   long long tmp_elems; // doubles of temporaries
 };
 
@@ -832,8 +832,8 @@ int build(int op, int cent, const cgx_array *dst, const cgx_array *srcs, const d
       s.dsy = d.n[0];
       s.dsz = (long long)d.n[0] * d.n[1];
       for (int k = 0; k < 3; ++k) s.doff[k] = 0;
-      b.st_ntiles = kind_tiles(s);
-      if (b.st_ntiles <= 0) return fail(CGX_EINVAL, "transfer: region too large");
+      b.st_ntiles[t] = kind_tiles(s);
+      if (b.st_ntiles[t] <= 0) return fail(CGX_EINVAL, "transfer: region too large");
     }
     d.kind = K_TIME;
     d.order = 0;
@@ -858,7 +858,7 @@ int launch_staged(Built &b, int fp, int *status, cudaStream_t s) {
   if (e != cudaSuccess) return cuda_fail(e, "cudaMallocAsync");
   bind_tmp(b, tmp);
   int rc = CGX_OK;
-  for (int t = 0; t < b.nst && rc == CGX_OK; ++t) rc = launch_pair(b.st[t], b.st_ntiles, fp, status, s);
+  for (int t = 0; t < b.nst && rc == CGX_OK; ++t) rc = launch_pair(b.st[t], b.st_ntiles[t], fp, status, s);
   if (rc == CGX_OK) rc = launch_pair(b.d, b.ntiles, fp, status, s);
   e = cudaFreeAsync(tmp, s);
   if (rc == CGX_OK && e != cudaSuccess) rc = cuda_fail(e, "cudaFreeAsync");
@@ -1001,7 +1001,7 @@ void batch_add_built(cgx_batch *b, const Built &x) {
     return;
   }
   const long long base = b->tmp_elems, npts = x.tmp_elems / x.nst;
-  for (int t = 0; t < x.nst; ++t) batch_push(b, x.st[t], 0, 0, x.st_ntiles, base + t * npts, -1);
+  for (int t = 0; t < x.nst; ++t) batch_push(b, x.st[t], 0, 0, x.st_ntiles[t], base + t * npts, -1);
   batch_push(b, x.d, x.bytes, x.points, x.ntiles, -1, base);
   b->nstage1 += x.nst;
   b->tmp_elems += x.tmp_elems;
