@@ -253,21 +253,19 @@ int row_units(const Desc &d) {
   return 4LL * ns * d.n[1] * d.n[2] < (1LL << 31) ? ns : 0;
 }
 
-// cuTensorMapEncodeTiled from the driver, found once; null without a driver
+// cuTensorMapEncodeTiled from the driver, found by the first caller while any
+// others wait for it; null without a driver
 PFN_cuTensorMapEncodeTiled_v12000 tma_encoder() {
-  static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
-  static bool tried = false;
-  if (!tried) {
-    tried = true;
+  static const PFN_cuTensorMapEncodeTiled_v12000 fn = [] {
     void *p = nullptr;
     cudaDriverEntryPointQueryResult q = cudaDriverEntryPointSymbolNotFound;
     if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &q) ==
             cudaSuccess &&
         q == cudaDriverEntryPointSuccess)
-      fn = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(p);
-    else
-      cudaGetLastError();
-  }
+      return reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(p);
+    cudaGetLastError();
+    return PFN_cuTensorMapEncodeTiled_v12000(nullptr);
+  }();
   return fn;
 }
 

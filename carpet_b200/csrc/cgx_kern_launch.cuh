@@ -1,6 +1,8 @@
 // cgx_kern_launch.cuh -- host launchers of one floating-point mode's
 // kernels; included once per mode by cgx_kern_f0.cu / cgx_kern_f1.cu.
 #pragma once
+#include <atomic>
+
 #include "cgx_kernels.cuh"
 
 namespace cgx {
@@ -137,7 +139,7 @@ int launch_tma_family(int variant, const Desc *d_descs, const CUtensorMap *d_map
 
 template <int FMA, class F, int NTL, int TK>
 int launch_box_v(const Desc &d, const CUtensorMap *maps, int ntiles, int *status, cudaStream_t s) {
-  static bool attr = false;
+  static std::atomic<bool> attr{false}; // plain calls come from any thread; setting it twice does no harm
   const size_t smem = sizeof(double) * TSmem<F, NTL, BOX_CFG>::total + 128; // + alignment slack
   if (!attr) {
     cudaError_t e = cudaFuncSetAttribute(k_tma_box<FMA, F, NTL, TK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
