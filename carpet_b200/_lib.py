@@ -46,6 +46,7 @@ lib.cgx_transfer.argtypes = [C.c_int, C.c_int, _P(cgx_array), _P(cgx_array), _P(
                              C.c_void_p]
 # a cgx_pair record, packed by carpet_b200.transfer
 lib.cgx_transfer_pair.argtypes = [C.c_char_p, C.c_void_p]
+lib.cgx_transfer_check.argtypes = [C.c_void_p]
 lib.cgx_copy.argtypes = [C.c_int, C.c_int, _P(cgx_array), _P(cgx_array), _i9, _i9, C.c_void_p,
                          C.c_void_p]
 lib.cgx_batch_add.argtypes = [C.c_void_p, C.c_int, C.c_int, _P(cgx_array), _P(cgx_array),

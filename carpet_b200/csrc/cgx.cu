@@ -14,6 +14,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <climits>
 #include <cmath>
 #include <cstdarg>
@@ -863,15 +864,51 @@ int launch_staged(Built &b, int fp, int *status, cudaStream_t s) {
   return rc;
 }
 
+constexpr int kMaxDevices = 64;
+
+// The status word of plain calls, one per device (cgx_transfer_check): a box
+// staged by TMA has a bounded wait, and a plain call has no object of its own
+// to keep the word in.  In host code this name only stands in for the symbol.
+static __device__ int g_plain_status;
+std::atomic<int *> g_plain_status_dev[kMaxDevices];
+
+// its address on the current device, looked up by the first call there; a
+// stream capture of the calling thread does not see the look-up
+int plain_status(int **out) {
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return cuda_fail(e, "cudaGetDevice");
+  if (dev < 0 || dev >= kMaxDevices) return fail(CGX_EINVAL, "device index %d out of range", dev);
+  int *p = g_plain_status_dev[dev].load();
+  if (!p) {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    void *q = nullptr;
+    e = cudaGetSymbolAddress(&q, g_plain_status);
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    if (e != cudaSuccess) return cuda_fail(e, "cudaGetSymbolAddress");
+    p = static_cast<int *>(q);
+    g_plain_status_dev[dev].store(p);
+  }
+  *out = p;
+  return CGX_OK;
+}
+
+// failure injection for the tests of the bounded device waits
+// (cgx_debug_skip_tma_plane)
+bool g_debug_skip_tma = false;
+
 // A box tiled for TMA.  Its tensor maps are encoded here, on each launch.
 int launch_box(const Desc &d, int ntiles, int fp, int *status, cudaStream_t s) {
   CUtensorMap maps[3] = {};
   Desc t = d;
   if (!encode_tma_maps(t, maps)) return fail(CGX_ECUDA, "transfer: a tensor map could not be encoded");
-  const int v = tma_variant(d);
+  if (!status)
+    if (int rc = plain_status(&status)) return rc;
+  const int u = tma_variant(d), v = u | (g_debug_skip_tma ? 1 << 30 : 0);
   const bool f = fp == CGX_FP_FMA;
-  if (v >= TV_TUNED) return klaunch_box_eno(f, v, d, maps, ntiles, status, s);
-  if (v / 4 >= 5) return f ? klaunch_box_f1_p1(v, d, maps, ntiles, status, s) : klaunch_box_f0_p1(v, d, maps, ntiles, status, s);
+  if (u >= TV_TUNED) return klaunch_box_eno(f, v, d, maps, ntiles, status, s);
+  if (u / 4 >= 5) return f ? klaunch_box_f1_p1(v, d, maps, ntiles, status, s) : klaunch_box_f0_p1(v, d, maps, ntiles, status, s);
   return f ? klaunch_box_f1_p0(v, d, maps, ntiles, status, s) : klaunch_box_f0_p0(v, d, maps, ntiles, status, s);
 }
 
@@ -899,10 +936,6 @@ const TmaLaunch kTmaLaunch[2][2][TMA_NCFG] = {{CGX_TMA_ROW(0, 0), CGX_TMA_ROW(0,
 int launch_map_capped(int fp, const Desc *d, const CUtensorMap *maps, const int2 *tmap,
                       const long long seg[NSEG + 1], const int *cfg, unsigned long long *counter, int *status,
                       cudaStream_t s);
-// failure injection for the tests of the bounded device waits
-// (cgx_debug_skip_tma_plane)
-bool g_debug_skip_tma = false;
-
 // with the batch's CTA caps in force for these launches only
 int launch_map(int fp, const Desc *d, const CUtensorMap *maps, const int2 *tmap,
                const long long seg[NSEG + 1], const int *cfg, unsigned long long *counter, int *status,
@@ -1075,6 +1108,18 @@ int cgx_transfer_pair(const cgx_pair *p, void *stream) {
   if (p->nsrc > 3) return fail(CGX_EINVAL, "transfer: a record holds at most 3 source timelevels");
   return cgx_transfer(p->op, p->cent, &p->dst, p->srcs, p->times, p->nsrc, p->dstbox, p->srcbox,
                       p->has_slab ? p->slab_offset : nullptr, p->time, p->order_space, p->order_time, stream);
+}
+
+int cgx_transfer_check(void *stream) {
+  int *word = nullptr, st = 0;
+  int rc = plain_status(&word);
+  if (rc) return rc;
+  cudaStream_t s = (cudaStream_t)stream;
+  cudaError_t e = cudaMemcpyAsync(&st, word, sizeof(int), cudaMemcpyDeviceToHost, s);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  if (e == cudaSuccess && st) e = cudaMemsetAsync(word, 0, sizeof(int), s);
+  if (e != cudaSuccess) return cuda_fail(e, "status read-back");
+  return st ? fail(st, "cgx_transfer: a bounded device wait gave up (status %d)", st) : CGX_OK;
 }
 
 int cgx_copy(int op, int cent, const cgx_array *dst, const cgx_array *src, const int dstbox[9],
@@ -1784,7 +1829,6 @@ constexpr size_t kNoAllocBytes = kNoAllocCounterOff + 256; // counter + status
 // its device address comes from cudaGetSymbolAddress, once per device.
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocBytes];
 
-constexpr int kMaxDevices = 64;
 unsigned char *g_noalloc_dev[kMaxDevices] = {nullptr};
 
 // Device address of the scratch on the current device; the first call on a

@@ -138,7 +138,7 @@ int launch_tma_family(int variant, const Desc *d_descs, const CUtensorMap *d_map
 }
 
 template <int FMA, class F, int NTL, int TK>
-int launch_box_v(const Desc &d, const CUtensorMap *maps, int ntiles, int *status, cudaStream_t s) {
+int launch_box_v(int variant, const Desc &d, const CUtensorMap *maps, int ntiles, int *status, cudaStream_t s) {
   static std::atomic<bool> attr{false}; // plain calls come from any thread; setting it twice does no harm
   const size_t smem = sizeof(double) * TSmem<F, NTL, BOX_CFG>::total + 128; // + alignment slack
   if (!attr) {
@@ -148,17 +148,17 @@ int launch_box_v(const Desc &d, const CUtensorMap *maps, int ntiles, int *status
   }
   BoxMaps m;
   for (int t = 0; t < 3; ++t) m.m[t] = maps[t];
-  k_tma_box<FMA, F, NTL, TK><<<ntiles, TMA_CFGS[BOX_CFG].nt, smem, s>>>(d, m, status);
+  k_tma_box<FMA, F, NTL, TK><<<ntiles, TMA_CFGS[BOX_CFG].nt, smem, s>>>(d, m, status, (variant >> 30 & 1) != 0);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? CGX_OK : cuda_error(e, "k_tma_box launch");
 }
 template <int FMA, class F>
 int launch_box_family(int variant, const Desc &d, const CUtensorMap *maps, int ntiles, int *status, cudaStream_t s) {
   switch (variant % 4) {
-  case 0: return launch_box_v<FMA, F, 1, T_NONE>(d, maps, ntiles, status, s);
-  case 1: return launch_box_v<FMA, F, 2, T_LIN>(d, maps, ntiles, status, s);
-  case 2: return launch_box_v<FMA, F, 3, T_QUAD>(d, maps, ntiles, status, s);
-  default: return launch_box_v<FMA, F, 3, T_ENO>(d, maps, ntiles, status, s);
+  case 0: return launch_box_v<FMA, F, 1, T_NONE>(variant, d, maps, ntiles, status, s);
+  case 1: return launch_box_v<FMA, F, 2, T_LIN>(variant, d, maps, ntiles, status, s);
+  case 2: return launch_box_v<FMA, F, 3, T_QUAD>(variant, d, maps, ntiles, status, s);
+  default: return launch_box_v<FMA, F, 3, T_ENO>(variant, d, maps, ntiles, status, s);
   }
 }
 

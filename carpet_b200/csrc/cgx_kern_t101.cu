@@ -17,7 +17,7 @@ int klaunch_tma_f1_p0_c1(int variant, const Desc *d, const CUtensorMap *maps, co
 // single boxes (k_tma_box)
 int klaunch_box_f1_p0(int variant, const Desc &d, const CUtensorMap *maps, int ntiles, int *status,
                       cudaStream_t s) {
-  switch (variant / 4) {
+  switch ((variant & ~(1 << 30)) / 4) {
   case 0: return kern::launch_box_family<1, VC<1>>(variant, d, maps, ntiles, status, s);
   case 1: return kern::launch_box_family<1, VC<3>>(variant, d, maps, ntiles, status, s);
   case 2: return kern::launch_box_family<1, VC<5>>(variant, d, maps, ntiles, status, s);

@@ -17,7 +17,7 @@ int klaunch_tma_f1_p1_c1(int variant, const Desc *d, const CUtensorMap *maps, co
 // single boxes (k_tma_box)
 int klaunch_box_f1_p1(int variant, const Desc &d, const CUtensorMap *maps, int ntiles, int *status,
                       cudaStream_t s) {
-  switch (variant / 4) {
+  switch ((variant & ~(1 << 30)) / 4) {
   case 5: return kern::launch_box_family<1, CC<2>>(variant, d, maps, ntiles, status, s);
   case 6: return kern::launch_box_family<1, CC<3>>(variant, d, maps, ntiles, status, s);
   case 7: return kern::launch_box_family<1, CC<4>>(variant, d, maps, ntiles, status, s);

@@ -16,10 +16,11 @@ int klaunch_tma_eno(int fp, int variant, const Desc *d, const CUtensorMap *maps,
 }
 int klaunch_box_eno(int fp, int variant, const Desc &d, const CUtensorMap *maps, int ntiles, int *status,
                     cudaStream_t s) {
+  const bool o2 = (variant & ~(1 << 30)) / 4 == 10;
   if (fp)
-    return variant / 4 == 10 ? kern::launch_box_family<1, CCENO<2>>(variant, d, maps, ntiles, status, s)
-                             : kern::launch_box_family<1, CCENO<3>>(variant, d, maps, ntiles, status, s);
-  return variant / 4 == 10 ? kern::launch_box_family<0, CCENO<2>>(variant, d, maps, ntiles, status, s)
-                           : kern::launch_box_family<0, CCENO<3>>(variant, d, maps, ntiles, status, s);
+    return o2 ? kern::launch_box_family<1, CCENO<2>>(variant, d, maps, ntiles, status, s)
+              : kern::launch_box_family<1, CCENO<3>>(variant, d, maps, ntiles, status, s);
+  return o2 ? kern::launch_box_family<0, CCENO<2>>(variant, d, maps, ntiles, status, s)
+            : kern::launch_box_family<0, CCENO<3>>(variant, d, maps, ntiles, status, s);
 }
 } // namespace cgx

@@ -446,7 +446,7 @@ struct BoxMaps {
 };
 template <int FMA, class F, int NTL, int TK>
 __global__ void __launch_bounds__(TMA_CFGS[BOX_CFG].nt, tma_blocks<F, NTL, TK, BOX_CFG>())
-    k_tma_box(const __grid_constant__ Desc d, const __grid_constant__ BoxMaps maps, int *status) {
+    k_tma_box(const __grid_constant__ Desc d, const __grid_constant__ BoxMaps maps, int *status, bool skip) {
   extern __shared__ __align__(128) double smraw[];
   const unsigned sbase = smem_u32(smraw);
   double *sm = smraw + ((((sbase + 127u) & ~127u) - sbase) >> 3);
@@ -456,7 +456,7 @@ __global__ void __launch_bounds__(TMA_CFGS[BOX_CFG].nt, tma_blocks<F, NTL, TK, B
     mbar_fence_init();
   }
   __syncthreads();
-  TmaRing ring{s_bars};
+  TmaRing ring{s_bars, 0u, skip}; // skip: failure injection
   prolong_tile<F, FMA, NTL, TK, BOX_CFG, true>(d, maps.m, (int)blockIdx.x, sm, ring, status);
 }
 

@@ -165,6 +165,13 @@ def copy_data(dst: Data, src: Data, dstbox, srcbox, op: int = OP_LAGRANGE, cent:
               stream)
 
 
+def check_transfers(stream=None):
+    """waits for the stream and raises if a bounded device wait of a plain call
+    (transfer_data, copy_data) on the current device gave up since the last
+    check, which leaves a destination incomplete (cgx_transfer_check)"""
+    check(lib.cgx_transfer_check(_stream(stream)))
+
+
 def find_source_timelevel(times, time, order_time, op):
     tl0, ntl = C.c_int(), C.c_int()
     ts = (C.c_double * len(times))(*times)

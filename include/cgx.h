@@ -103,7 +103,8 @@ const char *cgx_version(void);
  *   srcs[nsrc], times[nsrc]: source timelevels (same padext/bbox each);
  *   slab_offset: NULL or int[3], the islab offset of copy_3d (copy_3d.cc:57);
  *   stream: a cudaStream_t (NULL = default stream).
- * Asynchronous: returns after the launch.
+ * Asynchronous: returns after the launch.  cgx_transfer_check tells whether a
+ * bounded device wait gave up meanwhile.
  */
 int cgx_transfer(int op, int cent, const cgx_array *dst, const cgx_array *srcs,
                  const double *times, int nsrc, const int dstbox[9],
@@ -115,6 +116,14 @@ int cgx_transfer(int op, int cent, const cgx_array *dst, const cgx_array *srcs,
 int cgx_copy(int op, int cent, const cgx_array *dst, const cgx_array *src,
              const int dstbox[9], const int srcbox[9], const int *slab_offset,
              void *stream);
+
+/* Waits for the stream and returns the status of the plain calls
+ * (cgx_transfer, cgx_transfer_pair, cgx_copy) made on the current device since
+ * the last check: CGX_OK, or CGX_EDEVICE when the bounded wait of a large
+ * prolongation staged by tensor copies gave up, whose destination is then
+ * incomplete.  One word per device for all streams and threads; reading an
+ * error clears it. */
+int cgx_transfer_check(void *stream);
 
 /* The timelevel selection alone (gdata::find_source_timelevel). */
 int cgx_find_source_timelevel(const double *times, int ntimes, double time,
@@ -356,10 +365,11 @@ int cgx_chain_stats(const cgx_chain *c, int64_t *npairs, int64_t *ntiles, int64_
  * (a TMA copy landing on its mbarrier, a chain tile's dependency counter)
  * gives up after about 2^31 clock cycles (a second), records CGX_EDEVICE in
  * the launch's status word and lets the launch drain, so that the context
- * stays usable; the batch / chain check then reports CGX_EDEVICE.
+ * stays usable; the batch / chain / plain-call check then reports CGX_EDEVICE.
  *   cgx_debug_skip_tma_plane(1): the TMA prolongation kernels launched from
- *     now on never stage the first plane of each CTA's first tile, so that
- *     the wait for it runs out (0 restores normal operation);
+ *     now on (batched, or large single boxes) never stage the first plane of
+ *     each CTA's first tile, so that the wait for it runs out (0 restores
+ *     normal operation);
  *   cgx_chain_debug_hold(c, 1): the next cgx_chain_upload of c requires one
  *     more completed tile of every counter than exists, so that every
  *     dependency wait runs out (0 and a new upload restore it).
