@@ -218,20 +218,25 @@ struct PzCost { // of the candidates pz, pz / 2, ... 4 of a configuration
   static constexpr int NC = 5;
   int pz0, slots;
   double sum[NC] = {}, longest[NC] = {};
+  double tiles[NC] = {};
   explicit PzCost(int config) : pz0(TMA_CFGS[config].pz), slots(SM_COUNT * TMA_CFGS[config].mb) {}
   void add(const Desc &d) { // tiled in x and y
     const int zo = d.soff[2] & 1, W = stencil_width(d), n = d.n[2] + zo;
     for (int c = 0; c < NC && pz0 >> c >= 4; ++c) {
       const int pz = (ceil_div(n, ceil_div(n, pz0 >> c)) + 1) & ~1;
       const double cost = pz / 2 + W + 4;
-      sum[c] += (double)d.tiles[0] * d.tiles[1] * ceil_div(n, pz) * cost;
+      const double nt = (double)d.tiles[0] * d.tiles[1] * ceil_div(n, pz);
+      tiles[c] += nt;
+      sum[c] += nt * cost;
       longest[c] = std::max(longest[c], cost);
     }
   }
-  int best() const {
+  // at_once: tiles that all have a slot take the longest one's time
+  int best(bool at_once = false) const {
+    auto time = [&](int c) { return (at_once && tiles[c] <= slots ? 0.0 : sum[c] / slots) + longest[c]; };
     int b = 0;
     for (int c = 1; c < NC && pz0 >> c >= 4; ++c)
-      if (sum[c] / slots + longest[c] < sum[b] / slots + longest[b]) b = c;
+      if (time(c) < time(b)) b = c;
     return pz0 >> b;
   }
 };
@@ -751,10 +756,12 @@ int build_spatial(int op, int cent, const cgx_array *dst, const cgx_array *src,
   return fail(CGX_EINVAL, "transfer_p_r: mixed strides");
 }
 
-// One box-pair: gdata::transfer_data on one process + transfer_time.
+// One box-pair: gdata::transfer_data on one process + transfer_time.  Tiled to
+// be launched alone, or with tile = false left to a caller that tiles it as
+// one of a list (a pair that needs temporaries is tiled all the same).
 int build(int op, int cent, const cgx_array *dst, const cgx_array *srcs, const double *times,
           int nsrc, const int *dstbox_, const int *srcbox_, const int *slab, double time,
-          int order_space, int order_time, Built *out) {
+          int order_space, int order_time, Built *out, bool tile = true) {
   if (!dst || !srcs || !dstbox_ || !srcbox_) return fail(CGX_EINVAL, "transfer: null argument");
   if (op == CGX_OP_ERROR || op == CGX_OP_NONE)
     return fail(CGX_EINVAL, "transfer_data: operator is none/error");
@@ -841,8 +848,10 @@ int build(int op, int cent, const cgx_array *dst, const cgx_array *srcs, const d
     b.nst = ntl;
     b.tmp_elems = ntl * npts;
   }
-  b.ntiles = kind_tiles(d);
-  if (b.ntiles <= 0) return fail(CGX_EINVAL, "transfer: region too large");
+  if (tile) {
+    b.ntiles = kind_tiles(d);
+    if (b.ntiles <= 0) return fail(CGX_EINVAL, "transfer: region too large");
+  }
   *out = b;
   return CGX_OK;
 }
@@ -1876,42 +1885,51 @@ extern "C" int cgx_transfer_pairs_noalloc(const cgx_pair *pairs, int npairs, voi
   unsigned long long *d_counter = reinterpret_cast<unsigned long long *>(base + kNoAllocCounterOff);
   int *d_status = reinterpret_cast<int *>(base + kNoAllocCounterOff + sizeof(unsigned long long));
 
-  // Validate on the host into small stack chunks and copy each chunk into
-  // the scratch; cudaMemcpyAsync has staged pageable sources when it returns.
-  constexpr int kChunk = 16;
-  Desc hd[kChunk];
-  long long hp[kChunk];
+  // Validate on the host; the list's prolongations (the cp.async kernels'
+  // tiles) are cut in z by what they take together: 18 slabs of 64 x 12 x 52
+  // cut one by one took 50 us (3 waves of short tiles), 29 us so; 64 with three
+  // timelevels, 256 tiles that run at once uncut, 87 us against 97 us cut
+  std::vector<Desc> hd((size_t)npairs);
+  std::vector<long long> hp((size_t)npairs);
+  PzCost cost(PLAIN_CFG);
+  for (int i = 0; i < npairs; ++i) {
+    const cgx_pair &p = pairs[i];
+    if (p.nsrc < 1 || p.nsrc > 3) return fail(CGX_EINVAL, "pair %d: nsrc must be 1..3", i);
+    Built b;
+    rc = build(p.op, p.cent, &p.dst, p.srcs, p.times, p.nsrc, p.dstbox, p.srcbox,
+               p.has_slab ? p.slab_offset : nullptr, p.time, p.order_space, p.order_time, &b, false);
+    if (rc) return rc;
+    if (b.nst)
+      return fail(CGX_EUNSUPPORTED,
+                  "pair %d: a transfer through per-timelevel temporaries (restriction between "
+                  "timelevels, order_time 3 or 4) is not available without allocation", i);
+    if (b.d.kind == K_PROLONG_VC && b.d.order >= 7)
+      return fail(CGX_EUNSUPPORTED, "pair %d: vertex-centred order %d is not available without allocation", i,
+                  b.d.order);
+    Desc &d = hd[i] = b.d;
+    if (!is_stencil(d.kind)) {
+      hp[i] = stream_tiles(d, row_units(d));
+    } else if (prolong_xy(d, PLAIN_CFG)) {
+      cost.add(d);
+    } else {
+      return fail(CGX_EINVAL, "pair %d: region too large", i);
+    }
+  }
+  const int pz = cost.best(true);
   long long tiles = 0;
+  for (int i = 0; i < npairs; ++i) { // hp: tile counts -> first tiles
+    const long long nt = is_stencil(hd[i].kind) ? prolong_z(hd[i], PLAIN_CFG, pz) : hp[i];
+    if (nt <= 0 || nt >= (1LL << 31)) return fail(CGX_EINVAL, "pair %d: region too large", i);
+    hp[i] = tiles;
+    tiles += nt;
+  }
+  // cudaMemcpyAsync has staged pageable sources when it returns
+  constexpr int kChunk = 16;
   for (int i0 = 0; i0 < npairs; i0 += kChunk) {
     const int n = std::min(kChunk, npairs - i0);
-    for (int i = 0; i < n; ++i) {
-      const cgx_pair &p = pairs[i0 + i];
-      if (p.nsrc < 1 || p.nsrc > 3)
-        return fail(CGX_EINVAL, "pair %d: nsrc must be 1..3", i0 + i);
-      Built b;
-      rc = build(p.op, p.cent, &p.dst, p.srcs, p.times, p.nsrc, p.dstbox, p.srcbox,
-                 p.has_slab ? p.slab_offset : nullptr, p.time, p.order_space, p.order_time, &b);
-      if (rc) return rc;
-      if (b.nst)
-        return fail(CGX_EUNSUPPORTED,
-                    "pair %d: a transfer through per-timelevel temporaries (restriction between "
-                    "timelevels, order_time 3 or 4) is not available without allocation", i0 + i);
-      if (b.d.kind == K_PROLONG_VC && b.d.order >= 7)
-        return fail(CGX_EUNSUPPORTED,
-                    "pair %d: vertex-centred order %d is not available without allocation",
-                    i0 + i, b.d.order);
-      hd[i] = b.d;
-      hp[i] = tiles;
-      // the cp.async kernels' tiles; a list of many pairs fills the GPU with
-      // whole-length ones
-      if (is_stencil(b.d.kind))
-        b.ntiles = (int)(npairs > SM_COUNT / 8 ? prolong_tiles(hd[i], PLAIN_CFG, TMA_CFGS[PLAIN_CFG].pz)
-                                               : prolong_tiles_alone(hd[i], PLAIN_CFG));
-      tiles += b.ntiles;
-    }
-    cudaError_t e = cudaMemcpyAsync(d_descs + i0, hd, n * sizeof(Desc), cudaMemcpyHostToDevice, s);
+    cudaError_t e = cudaMemcpyAsync(d_descs + i0, &hd[i0], n * sizeof(Desc), cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess)
-      e = cudaMemcpyAsync(d_prefix + i0, hp, n * sizeof(long long), cudaMemcpyHostToDevice, s);
+      e = cudaMemcpyAsync(d_prefix + i0, &hp[i0], n * sizeof(long long), cudaMemcpyHostToDevice, s);
     if (e != cudaSuccess) return cuda_fail(e, "scratch upload");
   }
   // the work counter and the status word start at zero on every call
