@@ -77,7 +77,7 @@ struct Box {
 
 // The magic number and shift of div_magic (cgx_device.cuh) for divisor n:
 // l = ceil(log2 n), m = ceil(2^(31+l) / n), s = l - 1; m = 0 encodes n = 1.
-void division_magic(int n, unsigned *m, unsigned char *s) {
+void division_magic(int n, unsigned *m, int *s) {
   if (n <= 1) {
     *m = 0;
     *s = 0;
@@ -87,7 +87,7 @@ void division_magic(int n, unsigned *m, unsigned char *s) {
   while ((1LL << l) < n) ++l;
   const unsigned long long num = 1ULL << (31 + l); // l <= 31
   *m = (unsigned)((num + (unsigned)n - 1) / (unsigned)n);
-  *s = (unsigned char)(l - 1);
+  *s = l - 1;
 }
 
 struct Win { int lo0, hi0, lo1, hi1; };
@@ -199,8 +199,7 @@ long long prolong_z(Desc &d, int config, int pzmax) {
   const int stages = ceil_div(planes, fixed ? fixed : std::min(rpt / d.by, tls / (d.bx * d.by)));
   d.bz = (unsigned char)(fixed ? fixed : ceil_div(planes, stages));
   d.pz = (short)pz;
-  d.tiles[2] = ceil_div(d.n[2] + zo, pz);
-  return (long long)d.tiles[0] * d.tiles[1] * d.tiles[2];
+  return (long long)d.tiles[0] * d.tiles[1] * ceil_div(d.n[2] + zo, pz);
 }
 long long prolong_tiles(Desc &d, int config, int pzmax) {
   return prolong_xy(d, config) ? prolong_z(d, config, pzmax) : -1;
@@ -305,11 +304,10 @@ long long stream_tiles(Desc &d, int ns) {
     d.tiles[0] = ceil_div(d.n[0], CC5X);
     d.tiles[1] = ceil_div(d.n[1], CC5Y);
     d.pz = (long long)d.n[0] * d.n[1] * d.n[2] >= 1 << 16 ? 16 : 4;
-    d.tiles[2] = ceil_div(d.n[2], d.pz);
-    return (long long)d.tiles[0] * d.tiles[1] * d.tiles[2];
+    return (long long)d.tiles[0] * d.tiles[1] * ceil_div(d.n[2], d.pz);
   }
   d.tiles[0] = (int)((row * d.n[1] * d.n[2] + per - 1) / per);
-  d.tiles[1] = d.tiles[2] = 1;
+  d.tiles[1] = 1;
   division_magic((int)row, &d.mg[0], &d.sh[0]);
   division_magic(d.n[1], &d.mg[1], &d.sh[1]);
   return d.tiles[0];
