@@ -1283,9 +1283,15 @@ int cgx_batch_upload(cgx_batch *b, void *stream) {
       copied += b->points[i];
       narrow += dq[i].ns ? 0 : b->points[i];
     }
-  if (8 * narrow > copied)
-    for (int i : order)
-      if (dq[i].kind == K_COPY && dq[i].ns) ntq[i] = stream_tiles(dq[i], 0);
+  // Copies of three timelevels go by sectors from 5 * 2^19 copied points on: a
+  // thread's sectors follow one another, 12 loads at a time, which a GPU that is
+  // not full does not hide (0.5 million points in 64 regions 10.0 us by points,
+  // 10.4 us by sectors, 1.8 million in 4 regions 14.0 and 14.6, 2.2 million in
+  // 100 16.3 and 17.8; 2.7 million in 6 20.7 and 19.9, 7.7 million in 16 57 and
+  // 47 us).
+  for (int i : order)
+    if (dq[i].kind == K_COPY && dq[i].ns && (8 * narrow > copied || (dq[i].ntl > 2 && copied < 5 << 19)))
+      ntq[i] = stream_tiles(dq[i], 0);
   // Batches that copy more than L2 keeps fetch their destinations ahead: a
   // ghost sync of 25 grid functions of 129^3 (125 MB) 76.2 -> 72.0 us and the
   // five-level step, whose syncs of 60 MB each find nothing in L2,
