@@ -135,8 +135,9 @@ int ceil_div(int a, int b) { return (a + b - 1) / b; }
 // against 520 us), and for more timelevels, which are bound by their
 // arithmetic, only where they cost none (the boundary slabs of 129^3 levels:
 // 176 us with sector tiles, a tenth more tiles, against 168 us).
-// prolong_xy lays out x and y (false: no tile fits), prolong_z then z.
-bool prolong_xy(Desc &d, int config) {
+// prolong_xy lays out x and y (false: no tile fits) with at most rowcap coarse
+// rows to a tile, prolong_z then z.
+bool prolong_xy(Desc &d, int config, int rowcap = INT_MAX) {
   const TmaCfg &c = TMA_CFGS[config];
   const int W = stencil_width(d), ntl = std::min(3, std::max(1, (int)d.ntl));
   const int fixed = tma_planes(family_phases(d.kind, d.order), ntl); // planes per stage, or 0
@@ -148,7 +149,7 @@ bool prolong_xy(Desc &d, int config) {
   };
   auto rows = [&](XTiles x) { // the rest of a choice of x tiles
     x.bx = tma_bx(x.nbx, W);
-    const int rmax = std::min(c.nt / x.ptx, std::min(rpt, tls / x.bx) / std::max(1, fixed) - W);
+    const int rmax = std::min({rowcap, c.nt / x.ptx, std::min(rpt, tls / x.bx) / std::max(1, fixed) - W});
     if (rmax < 1) return x.ny = 0, x;
     const int nty = ceil_div(d.n[1] + yo, 2 * rmax);
     x.nx = ceil_div(d.n[0] + x.xo, x.xw);
@@ -239,11 +240,21 @@ struct PzCost { // of the candidates pz, pz / 2, ... 4 of a configuration
     return pz0 >> b;
   }
 };
-long long prolong_tiles_alone(Desc &d, int config) { // one descriptor launched alone
+// One descriptor launched alone.  One that has no tile for every SM is cut in y
+// too, as long as each keeps an SM of its own: a thin box is a handful of tiles,
+// whose rows' threads share one SM's issue slots (33 x 33 x 3 of order 5 with
+// one and three timelevels, 3 tiles: 9.0 and 17.4 us, with 51 tiles 5.3 and
+// 8.5; 128 x 128 x 2, 32 tiles: 7.7 and 16.0, with 128 6.3 and 10.3, with 256
+// 9.5 and 9.4).
+long long prolong_tiles_alone(Desc &d, int config) {
   if (!prolong_xy(d, config)) return -1;
   PzCost c(config);
   c.add(d);
-  return prolong_z(d, config, c.best());
+  const int pz = c.best();
+  const long long nt = prolong_z(d, config, pz), fit = SM_COUNT / (nt / d.tiles[1]);
+  if (fit <= d.tiles[1]) return nt;
+  prolong_xy(d, config, ceil_div(d.n[1] + (d.soff[1] & 1), 2 * (int)fit));
+  return prolong_z(d, config, pz);
 }
 
 // Units per row of a copy (Sector, cgx_device.cuh): those of the most sectors
