@@ -105,21 +105,6 @@ def _array_fields(d: Data):
     return (d.tensor.data_ptr(), px, py, pz, *d.extent)
 
 
-def _nine(dst, srcs, times, dstbox, srcbox, slab_offset):
-    """every box and extent has nine numbers, a slab offset three, and there
-    is a time per source: the record only checks their sum.  False for what
-    has no length (an iterator), which is left as it is."""
-    try:
-        if len(dstbox) != 9 or len(srcbox) != 9 or len(dst.extent) != 9 or len(times) < len(srcs):
-            return False
-        for s in srcs:
-            if len(s.extent) != 9:
-                return False
-        return slab_offset is None or len(slab_offset) == 3
-    except TypeError:
-        return False
-
-
 def _raw_stream(stream):
     if stream is None:
         return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
@@ -131,17 +116,23 @@ def _transfer(op, cent, dst, srcs, times, dstbox, srcbox, slab_offset, time, ord
     call costs its host thread 7 us that way, of which the launch is 2.3,
     against 15 us with a ctypes object per argument."""
     n = len(srcs)
-    if 1 <= n <= 3 and _nine(dst, srcs, times, dstbox, srcbox, slab_offset):
-        try:
+    try:
+        # a record checks only the sum of the lengths; an iterator, which has
+        # none, is left whole (an extent of another length would put a pointer
+        # into an index and does not pack)
+        if 1 <= n <= 3 and len(dstbox) == len(srcbox) == 9 and len(times) >= n and (
+                slab_offset is None or len(slab_offset) == 3):
             pair = _PAIR.pack(
                 op, cent, *_array_fields(dst), *[f for s in srcs for f in _array_fields(s)],
                 *(_NO_ARRAY * (3 - n)), *times[:n], *((0.0,) * (3 - n)), n, *dstbox, *srcbox,
                 *((0, 0, 0, 0) if slab_offset is None else (1, *slab_offset)), time, order_space, order_time)
-        except (struct.error, TypeError):
-            pair = None  # numbers that are not integers as they stand
-        if pair is not None:
-            check(lib.cgx_transfer_pair(pair, _raw_stream(stream)))
-            return
+        else:
+            pair = None
+    except (struct.error, TypeError):
+        pair = None  # numbers that are not integers as they stand
+    if pair is not None:
+        check(lib.cgx_transfer_pair(pair, _raw_stream(stream)))
+        return
     d = dst.cgx()
     arr = _arrays(srcs)
     ts = (C.c_double * len(times))(*times)
