@@ -332,8 +332,11 @@ int kind_tiles(Desc &d) {
   long long tot = 1;
   if (prol) {
     // a box's tensor maps cost the call about 1 us per timelevel: staged by
-    // TMA from 2^18 source values on (161^3, order 5: 37 -> 16 us a call; a
-    // slab of 64 x 12 x 52 with three timelevels 18.0 against 17.3 us)
+    // TMA from 2^21 point-timelevels on (161^3, order 5: 37 -> 16 us a call; a
+    // slab of 64 x 12 x 52 with three timelevels 18.0 against 17.3 us).  The
+    // line lies above where the forms meet: 64^3, 2^18 points, 8.4 us by TMA
+    // and 10.5 us by plain loads, 128 x 128 x 64, 2^20, 8.5 and 15.7, 129^3 just
+    // above it 10.6 and 20.8; 64 x 32 x 32, 2^16, 11.8 and 10.9
     const bool big = (long long)d.n[0] * d.n[1] * d.n[2] * d.ntl >= 8LL << 18;
     const int cfg = big && tma_addressable(d) ? BOX_CFG : PLAIN_CFG;
     tot = prolong_tiles_alone(d, cfg);
@@ -1286,8 +1289,11 @@ int cgx_batch_upload(cgx_batch *b, void *stream) {
   for (int i : order)
     if (is_stencil(dq[i].kind)) by_variant[tma_addressable(dq[i]) ? tma_variant(dq[i]) : -1].push_back(i);
   // Copies go by sectors where hardly any of the batch's copied points lie in
-  // narrow rows: a ghost sync, a third of whose points do, stays one kernel
-  // (with two, its halves would be forked and joined at every phase).
+  // narrow rows: a ghost sync, a third of whose points do, stays one kernel.
+  // With two, forked and joined, the sync of a 129^3 level in 8 components took
+  // 23.4 us against 16.8 us with 4 grid functions, 23 to 26 against 20.9 with 8,
+  // 42.3 against 45.4 with 16, 70.9 against 72.0 with 25 (the five-level step
+  // 7.15 against 7.21 ms).
   long long narrow = 0, copied = 0;
   for (int i : order)
     if (dq[i].kind == K_COPY) {
@@ -1304,10 +1310,10 @@ int cgx_batch_upload(cgx_batch *b, void *stream) {
     if (dq[i].kind == K_COPY && dq[i].ns && (8 * narrow > copied || (dq[i].ntl > 2 && copied < 5 << 19)))
       ntq[i] = stream_tiles(dq[i], 0);
   // Batches that copy more than L2 keeps fetch their destinations ahead: a
-  // ghost sync of 25 grid functions of 129^3 (125 MB) 76.2 -> 72.0 us and the
-  // five-level step, whose syncs of 60 MB each find nothing in L2,
-  // 7.54 -> 7.24 ms; a sync of 8 (40 MB), its arrays in L2, took 22.0 instead
-  // of 20.6 us.
+  // ghost sync of 25 grid functions of 129^3 (125 MB) 76.2 us without and 72.1
+  // with it, the five-level step, whose syncs of 60 MB each find nothing in L2,
+  // 7.50 and 7.16 ms; a sync of 8 (40 MB), its arrays in L2, takes 20.9 us
+  // without and 22.9 with.
   for (int i : order) dq[i].ahead = dq[i].kind == K_COPY && 16 * copied >= 48 << 20;
   for (const auto &kv : by_variant) {
     const int cfg = kv.first >= 0 ? tma_cfg(kv.first, b->tma_cfg[kv.first]) : PLAIN_CFG;

@@ -502,7 +502,7 @@ __device__ __forceinline__ void unflatten(const D &d, unsigned p, int &i, int &j
 }
 
 // Unit p of the region's destination rows, the rows' first and last sectors
-// whole: its row, and the x (-7 .. n[0] + 6) of its first half sector, which
+// whole: its row, and the x (-3 .. n[0] + 4) of its first half sector, which
 // starts on 16 bytes; the other half lies four points further.
 struct Sector {
   int x, j, k;
@@ -949,9 +949,12 @@ __device__ __forceinline__ void restrict_cc3_tile(const D &d, int tile, int lid)
 // tile: about 100 operations and 30 loads of 16 bytes a point, where a point on
 // its own takes 473 and 108 and was bound by L1 (96 uneven regions of 8-32
 // coarse points a side: 246 us, two points sharing planes 103 us, this form
-// 57 us; beside the other restrictions of such a batch 189 -> 59 us in all).
-// Small regions take short tiles (pz 4), which run at once; large ones 16,
-// with fewer halo planes.
+// 57 us; a batch of all three restrictions, a third of the regions each, 187 -> 81
+// us a call).
+// Regions below 2^16 coarse points take short tiles (pz 4), which run at once.
+// Larger ones take 16, with fewer halo planes, which has not paid where it was
+// measured since: 96 regions of 64-96 points a side 315 us against 311 us with
+// short tiles, 8 of them 68 against 35.
 constexpr int CC5X = 16, CC5Y = 8;
 template <int FMA, int LANES, class D>
 __device__ __forceinline__ void restrict_cc5_tile(const D &d, int tile, int lid) {
